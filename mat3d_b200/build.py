@@ -19,10 +19,11 @@ LIB = os.path.join(HERE, "libmat3d_b200.so")
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a",
     "-O3", "-lineinfo", "-std=c++17",
-    "-Xcompiler", "-fPIC", "-shared",
+    "-Xcompiler", "-fPIC", "-shared", "--threads", "0",  # one compiler per source at a time
 ]
 
-SOURCES = [os.path.join(CSRC, "solver.cu"), os.path.join(CSRC, "noalloc.cu"), os.path.join(CSRC, "compat.cpp"),
+SOURCES = [os.path.join(CSRC, "solver.cu"), os.path.join(CSRC, "generic_r31.cu"),
+           os.path.join(CSRC, "generic_r13.cu"), os.path.join(CSRC, "noalloc.cu"), os.path.join(CSRC, "compat.cpp"),
            os.path.join(CSRC, "batch.cpp"), os.path.join(CSRC, "serve.cpp"),
            os.path.join(CSRC, "solver2d.cu"), os.path.join(CSRC, "rec.cu"), os.path.join(CSRC, "rec_compat.cpp")]
 DEPS = SOURCES + [os.path.join(CSRC, f) for f in os.listdir(CSRC)] + [

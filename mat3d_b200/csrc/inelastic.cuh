@@ -302,7 +302,7 @@ __global__ void k_constitutive(EpiConstitutive<T> epi, const Ctl* ctl, double* p
 // Increment commit (export_homogen_var :722-746 then update_old_Variable
 // :693-719): sums of eps_t, sig (6), sig_eff (J2) or d (ed), eps_p; then
 // eps_p += dp where phi > 0, sig_old = sig, eps extrapolation.
-__global__ void k_commit(InelasticPtrs<double> p, double* eps_old_w, double* sig_old_w, double* ep_w, int t_comp,
+static __global__ void k_commit(InelasticPtrs<double> p, double* eps_old_w, double* sig_old_w, double* ep_w, int t_comp,
                          double* partials) {
     extern __shared__ __align__(16) char smem_raw[];
     double* red = (double*)smem_raw;
@@ -384,7 +384,7 @@ __device__ __forceinline__ double prodv(const double* a, const double* b) {
 // E = k S0 X0 - S0 <sig> + <eps>.  S0 is isotropic: passed as its 6x6 in aux2.
 __device__ __forceinline__ void policy_j2(Ctl& c, const double* tot, int policy, double V, const double* S0m);
 
-__global__ void k_finalize_j2(Ctl* ctl, const double* __restrict__ partials, int NS, int nblk, int policy, double V,
+static __global__ void k_finalize_j2(Ctl* ctl, const double* __restrict__ partials, int NS, int nblk, int policy, double V,
                               const double* __restrict__ S0m) {
     const int b = blockIdx.x;
     if (ctl[b].done) return;

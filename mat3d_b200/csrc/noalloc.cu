@@ -265,10 +265,10 @@ extern "C" int m3d_thermal_solve_noalloc(int Nx, int Ny, int Nz, double km, doub
     {
         std::lock_guard<std::mutex> lk(g_noalloc_mu);  // kernel attributes are per device
         if (!g_noalloc_attrs[dev]) {
-            allow_dyn(k_zfwd<double, C, ProMat<double, C>>);
-            allow_dyn(k_ypass<double>);
-            allow_dyn(k_xturn<double, C, SpecGreen<double, C>>);
-            allow_dyn(k_zinv<double, C, EpiEM<double, C>, FinLinear>);
+            allow_dyn(k_zfwd<double, C, ProMat<double, C>, 5>);
+            allow_dyn(k_ypass<double, 5>);
+            allow_dyn(k_xturn<double, C, SpecGreen<double, C>, 5>);
+            allow_dyn(k_zinv<double, C, EpiEM<double, C>, FinLinear, 5>);
             g_noalloc_attrs[dev] = true;
         }
     }
@@ -277,11 +277,11 @@ extern "C" int m3d_thermal_solve_noalloc(int Nx, int Ny, int Nz, double km, doub
     const double2* twz = tw + Nx + Ny;
     for (;;) {
         for (int k = 0; k < 8; ++k) {
-            k_zfwd<double, C, ProMat<double, C>><<<dim3(zblk, 1), 256, zsmem, stream>>>(g, pz, twz, spec, pro, ctl, G, part);
-            k_ypass<double><<<dim3(Nx * ntzy, C), 256, ysmem, stream>>>(g, py, twy, spec, TZy, C, -1, ctl);
-            k_xturn<double, C, SpecGreen<double, C>><<<dim3(Ny * ntzx, 1), 256, xsmem, stream>>>(g, px, twx, spec, TZx, sg, ctl, part);
-            k_ypass<double><<<dim3(Nx * ntzy, C), 256, ysmem, stream>>>(g, py, twy, spec, TZy, C, +1, ctl);
-            k_zinv<double, C, EpiEM<double, C>, FinLinear><<<dim3(zblk, 1), 256, zsmem, stream>>>(g, pz, twz, spec, epi, ctl, G, part, fin);
+            k_zfwd<double, C, ProMat<double, C>, 5><<<dim3(zblk, 1), 256, zsmem, stream>>>(g, pz, twz, spec, pro, ctl, G, part);
+            k_ypass<double, 5><<<dim3(Nx * ntzy, C), 256, ysmem, stream>>>(g, py, twy, spec, TZy, C, -1, ctl);
+            k_xturn<double, C, SpecGreen<double, C>, 5><<<dim3(Ny * ntzx, 1), 256, xsmem, stream>>>(g, px, twx, spec, TZx, sg, ctl, part);
+            k_ypass<double, 5><<<dim3(Nx * ntzy, C), 256, ysmem, stream>>>(g, py, twy, spec, TZy, C, +1, ctl);
+            k_zinv<double, C, EpiEM<double, C>, FinLinear, 5><<<dim3(zblk, 1), 256, zsmem, stream>>>(g, pz, twz, spec, epi, ctl, G, part, fin);
         }
         NA_CUDA(cudaGetLastError());
         NA_CUDA(cudaMemcpyAsync(&hc, ctl, sizeof(hc), cudaMemcpyDeviceToHost, stream));

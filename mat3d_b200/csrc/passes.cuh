@@ -128,7 +128,7 @@ __device__ __forceinline__ char* align_up(char* p, int a) {
 // z forward: prologue (per voxel: C input values) -> pairs of real lines packed
 // as one complex line -> FFT along z -> split into two half spectra.
 // ============================================================================
-template <typename T, int C, class Pro>
+template <typename T, int C, class Pro, int MaxR>
 __global__ void __launch_bounds__(256) k_zfwd(GridDims g, LinePlan pz, const typename Cx<T>::t* __restrict__ twz,
                                               typename Cx<T>::t* __restrict__ spec, Pro pro, const Ctl* __restrict__ ctl,
                                               int G, double* partials) {
@@ -169,7 +169,7 @@ __global__ void __launch_bounds__(256) k_zfwd(GridDims g, LinePlan pz, const typ
     }
     __syncthreads();
     LineLayout L{nl, 1, 0, Nz, 1, false};
-    C2* R = fft_lines<C2>(A, B, tw, pz, L, -1);
+    C2* R = fft_lines<C2, MaxR>(A, B, tw, pz, L, -1);
 
     const int Hz = g.Hz, Hzp = g.Hzp;
     for (int i = threadIdx.x; i < nl * Hzp; i += blockDim.x) {
@@ -196,7 +196,7 @@ __global__ void __launch_bounds__(256) k_zfwd(GridDims g, LinePlan pz, const typ
 // y pass (forward sign -1 or inverse +1), in place on the half spectrum.
 // CTA = one x, TZ consecutive kz columns, one (batch, component).
 // ============================================================================
-template <typename T>
+template <typename T, int MaxR>
 __global__ void __launch_bounds__(256) k_ypass(GridDims g, LinePlan py, const typename Cx<T>::t* __restrict__ twy,
                                                typename Cx<T>::t* __restrict__ spec, int TZ, int C, int sign,
                                                const Ctl* __restrict__ ctl) {
@@ -219,7 +219,7 @@ __global__ void __launch_bounds__(256) k_ypass(GridDims g, LinePlan py, const ty
     }
     __syncthreads();
     LineLayout L{TZ, TZ, 1, 0, TZ, true};
-    C2* R = fft_lines<C2>(A, B, tw, py, L, sign);
+    C2* R = fft_lines<C2, MaxR>(A, B, tw, py, L, sign);
     for (int i = threadIdx.x; i < Ny * TZ; i += blockDim.x) {
         const int y = i / TZ, col = i - y * TZ;
         if (kz0 + col < Hzp) base[(long long)y * Hzp + col] = R[i];
@@ -231,7 +231,7 @@ __global__ void __launch_bounds__(256) k_ypass(GridDims g, LinePlan py, const ty
 //   forward FFT along x -> spectral op per mode (Green operator, k=0 value,
 //   optional reductions) -> inverse FFT along x (when Spec::kInverse).
 // ============================================================================
-template <typename T, int C, class Spec>
+template <typename T, int C, class Spec, int MaxR>
 __global__ void __launch_bounds__(256) k_xturn(GridDims g, LinePlan px, const typename Cx<T>::t* __restrict__ twx,
                                                typename Cx<T>::t* __restrict__ spec, int TZ, Spec op,
                                                const Ctl* __restrict__ ctl, double* partials) {
@@ -257,7 +257,7 @@ __global__ void __launch_bounds__(256) k_xturn(GridDims g, LinePlan px, const ty
     }
     __syncthreads();
     LineLayout L{C * TZ, TZ, 1, Nx * TZ, TZ, true};
-    C2* R = fft_lines<C2>(A, B, tw, px, L, -1);
+    C2* R = fft_lines<C2, MaxR>(A, B, tw, px, L, -1);
     C2* S = (R == A) ? B : A;
 
     double acc[Spec::NSUM > 0 ? Spec::NSUM : 1] = {};
@@ -279,7 +279,7 @@ __global__ void __launch_bounds__(256) k_xturn(GridDims g, LinePlan px, const ty
     }
     if constexpr (Spec::kInverse) {
         __syncthreads();
-        C2* Q = fft_lines<C2>(R, S, tw, px, L, +1);
+        C2* Q = fft_lines<C2, MaxR>(R, S, tw, px, L, +1);
         for (int i = threadIdx.x; i < C * Nx * TZ; i += blockDim.x) {
             const int col = i % TZ, r = i / TZ;
             const int x = r % Nx, c = r / Nx;
@@ -294,7 +294,7 @@ __global__ void __launch_bounds__(256) k_xturn(GridDims g, LinePlan px, const ty
 // Nyquist imaginary parts dropped, which is FFTW's c2r rule) -> inverse FFT ->
 // real parts / imaginary parts are the two real lines -> epilogue per voxel.
 // ============================================================================
-template <typename T, int C, class Epi, class Fin>
+template <typename T, int C, class Epi, class Fin, int MaxR>
 __global__ void __launch_bounds__(256) k_zinv(GridDims g, LinePlan pz, const typename Cx<T>::t* __restrict__ twz,
                                               const typename Cx<T>::t* __restrict__ spec, Epi epi, Ctl* ctl, int G,
                                               double* partials, Fin fin) {
@@ -333,7 +333,7 @@ __global__ void __launch_bounds__(256) k_zinv(GridDims g, LinePlan pz, const typ
     }
     __syncthreads();
     LineLayout L{nl, 1, 0, Nz, 1, false};
-    C2* R = fft_lines<C2>(A, B, tw, pz, L, +1);
+    C2* R = fft_lines<C2, MaxR>(A, B, tw, pz, L, +1);
 
     const T invV = (T)(1.0 / (double)g.V);
     double acc[Epi::NSUM > 0 ? Epi::NSUM : 1] = {};

@@ -28,10 +28,16 @@
 #include "passes_fast.cuh"
 #include "passes_slab.cuh"
 #include "fft_plan.hpp"
+#include "generic_launch.cuh"
 
 #include <cudaTypedefs.h>
 
 using namespace m3d;
+
+namespace m3d {
+M3D_GEN_ALL(extern, 13)
+M3D_GEN_ALL(extern, 31)
+}  // namespace m3d
 
 namespace {
 
@@ -109,27 +115,6 @@ Mat diag(int n, double v) {
     return o;
 }
 
-
-// Let a kernel use all dynamic shared memory left next to its static arrays
-// (227 KB per block on sm_100 in total).
-// Done once per kernel and device; safe to call from several host threads.
-std::mutex g_attr_mu;
-std::set<std::pair<int, const void*>> g_attr_done;
-template <class K>
-void allow_smem(K kernel) {
-    int dev = 0;
-    cudaGetDevice(&dev);
-    {
-        std::lock_guard<std::mutex> lk(g_attr_mu);
-        if (!g_attr_done.insert(std::make_pair(dev, (const void*)kernel)).second) return;
-    }
-    cudaFuncAttributes a;
-    if (cudaFuncGetAttributes(&a, kernel) == cudaSuccess) {
-        const int maxdyn = 227 * 1024 - (int)a.sharedSizeBytes;
-        cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, maxdyn);
-    }
-    (void)cudaGetLastError();  // an unsupported request must not surface at the next launch check
-}
 
 int even_up(int v) { return (v + 1) & ~1; }
 
@@ -622,8 +607,10 @@ void m3d_solver::pass_zfwd(Pro pro, Ctl* ctl, typename Cx<T>::t* sp) {
         const int Gl = G<T>();
         const int zblk = (int)((g.NL + Gl - 1) / Gl);
         const size_t zsmem = (size_t)Nz * sizeof(C2) + 2 * (size_t)(Gl / 2) * CC * Nz * sizeof(C2) + 16 + 32 * 32 * 8 + extra;
-        allow_smem(k_zfwd<T, CC, Pro>);
-        k_zfwd<T, CC, Pro><<<dim3(zblk, gridB()), 256, zsmem, stream>>>(g, pz, tw<T>(2), sp, pro, ctl, Gl, d_part);
+        with_radix(pz, [&](auto r) {
+            gen_zfwd<decltype(r)::value, T, CC, Pro>(dim3(zblk, gridB()), zsmem, stream, g, pz, tw<T>(2), sp, pro, ctl, Gl,
+                                                     d_part);
+        });
     }
     st.kernel_launches += 1;
 }
@@ -720,8 +707,9 @@ void m3d_solver::pass_y(int sign, int CC, Ctl* ctl, typename Cx<T>::t* sp) {
         const int tzy = TZy<T>();
         const size_t ysmem = (size_t)Ny * sizeof(C2) + 2 * (size_t)Ny * tzy * sizeof(C2);
         const int ntzy = (g.Hzp + tzy - 1) / tzy;
-        allow_smem(k_ypass<T>);
-        k_ypass<T><<<dim3(Nx * ntzy, CC * gridB()), 256, ysmem, stream>>>(g, py, tw<T>(1), sp, tzy, CC, sign, ctl);
+        with_radix(py, [&](auto r) {
+            gen_y<decltype(r)::value, T>(dim3(Nx * ntzy, CC * gridB()), ysmem, stream, g, py, tw<T>(1), sp, tzy, CC, sign, ctl);
+        });
     }
     st.kernel_launches += 1;
 }
@@ -797,8 +785,9 @@ int m3d_solver::pass_x(Spec op, Ctl* ctl, typename Cx<T>::t* sp) {
         const size_t xsmem = (size_t)Nx * sizeof(C2) + 2 * (size_t)CC * Nx * tzx * sizeof(C2) + 16 + 32 * 32 * 8;
         const int ntzx = (g.Hzp + tzx - 1) / tzx;
         nblk = Ny * ntzx;
-        allow_smem(k_xturn<T, CC, Spec>);
-        k_xturn<T, CC, Spec><<<dim3(nblk, gridB()), 256, xsmem, stream>>>(g, px, tw<T>(0), sp, tzx, op, ctl, d_part);
+        with_radix(px, [&](auto r) {
+            gen_x<decltype(r)::value, T, CC, Spec>(dim3(nblk, gridB()), xsmem, stream, g, px, tw<T>(0), sp, tzx, op, ctl, d_part);
+        });
     }
     st.kernel_launches += 1;
     return nblk;
@@ -821,8 +810,10 @@ int m3d_solver::pass_zinv(Epi epi, Ctl* ctl, typename Cx<T>::t* sp, Fin fin) {
         const int Gl = G<T>();
         nblk = (int)((g.NL + Gl - 1) / Gl);
         const size_t zsmem = (size_t)Nz * sizeof(C2) + 2 * (size_t)(Gl / 2) * CC * Nz * sizeof(C2) + 16 + 32 * 32 * 8 + extra;
-        allow_smem(k_zinv<T, CC, Epi, Fin>);
-        k_zinv<T, CC, Epi, Fin><<<dim3(nblk, gridB()), 256, zsmem, stream>>>(g, pz, tw<T>(2), sp, epi, ctl, Gl, d_part, fin);
+        with_radix(pz, [&](auto r) {
+            gen_zinv<decltype(r)::value, T, CC, Epi, Fin>(dim3(nblk, gridB()), zsmem, stream, g, pz, tw<T>(2), sp, epi, ctl, Gl,
+                                                          d_part, fin);
+        });
     }
     st.kernel_launches += 1;
     return nblk;

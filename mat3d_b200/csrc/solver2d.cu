@@ -27,6 +27,7 @@
 #include "../../include/mat3d_b200.h"
 #include "fft_plan.hpp"
 #include "fft_smem.cuh"
+#include "generic_launch.cuh"
 
 using namespace m3d;
 
@@ -89,7 +90,8 @@ __device__ __forceinline__ void cp_wait_all() { asm volatile("cp.async.wait_grou
 // iteration: eps = result / xy (FFTBCKWRD_epsilon :140-145).
 // (nbuf = 2 for the longest rows, whose third buffer does not fit: each tile
 // is then fetched after the previous one is stored)
-__global__ void k2d_rows(double2* __restrict__ buf, double2* __restrict__ eps, const double2* __restrict__ twy,
+template <int MaxR>
+__global__ void __launch_bounds__(256) k2d_rows(double2* __restrict__ buf, double2* __restrict__ eps, const double2* __restrict__ twy,
                          LinePlan py, int G, int nlines, int sign, long long xy, int nbuf) {
     extern __shared__ __align__(16) char smem_raw[];
     const int Ny = py.n;
@@ -128,7 +130,7 @@ __global__ void k2d_rows(double2* __restrict__ buf, double2* __restrict__ eps, c
             if (nxt < ntiles) fetch(S[f], nxt);
             cp_commit();
         }
-        double2* r = fft_lines(S[d], S[d == 2 ? 0 : d + 1], tw, py, L, sign);
+        double2* r = fft_lines<double2, MaxR>(S[d], S[d == 2 ? 0 : d + 1], tw, py, L, sign);
         const long long v0 = (long long)tile * tsz;
         const int valid = valid_of(tile);
         if (eps) {
@@ -146,7 +148,8 @@ __global__ void k2d_rows(double2* __restrict__ buf, double2* __restrict__ eps, c
 
 // Column turnaround: TZ consecutive columns y of all Nx rows and 3 components;
 // forward FFT along x, -Gamma0 : tau^ per mode (k = 0 -> E * xy), inverse FFT.
-__global__ void k2d_cols(double2* __restrict__ buf, const double2* __restrict__ twx, LinePlan px, int Ny, int TZ,
+template <int MaxR>
+__global__ void __launch_bounds__(256) k2d_cols(double2* __restrict__ buf, const double2* __restrict__ twx, LinePlan px, int Ny, int TZ,
                          Consts2D k, long long xy) {
     extern __shared__ __align__(16) char smem_raw[];
     const int Nx = px.n;
@@ -162,7 +165,7 @@ __global__ void k2d_cols(double2* __restrict__ buf, const double2* __restrict__ 
     }
     __syncthreads();
     LineLayout L{3 * TZ, TZ, 1, Nx * TZ, TZ, false};
-    double2* r = fft_lines(A, B, tw, px, L, -1);
+    double2* r = fft_lines<double2, MaxR>(A, B, tw, px, L, -1);
     double2* o = (r == A) ? B : A;
     // Green operator (setGF :49-103, multiplyGF :105-138)
     for (int i = threadIdx.x; i < Nx * TZ; i += blockDim.x) {
@@ -197,7 +200,7 @@ __global__ void k2d_cols(double2* __restrict__ buf, const double2* __restrict__ 
         for (int c = 0; c < 3; ++c) o[(c * Nx + x) * TZ + tz] = u[c];
     }
     __syncthreads();
-    double2* s = fft_lines(o, r, tw, px, L, +1);
+    double2* s = fft_lines<double2, MaxR>(o, r, tw, px, L, +1);
     for (int i = threadIdx.x; i < 3 * Nx * TZ; i += blockDim.x) {
         const int tz = i % TZ, cx = i / TZ, x = cx % Nx, c = cx / Nx;
         const int y = y0 + tz;
@@ -292,9 +295,15 @@ struct m3d_solver2d {
         const int nb = 592;
         k2d_pointwise<<<nb, 256, 0, stream>>>(eps, sig, buf, phase, k, xy);
         const int nlines = 3 * Nx;
-        k2d_rows<<<rows_grid, 256, rows_smem(), stream>>>(buf, nullptr, twy, py, G, nlines, -1, xy, rows_nbuf);
-        k2d_cols<<<(Ny + TZ - 1) / TZ, 256, cols_smem(), stream>>>(buf, twx, px, Ny, TZ, k, xy);
-        k2d_rows<<<rows_grid, 256, rows_smem(), stream>>>(buf, eps, twy, py, G, nlines, +1, xy, rows_nbuf);
+        with_radix(py, [&](auto r) {
+            k2d_rows<decltype(r)::value><<<rows_grid, 256, rows_smem(), stream>>>(buf, nullptr, twy, py, G, nlines, -1, xy, rows_nbuf);
+        });
+        with_radix(px, [&](auto r) {
+            k2d_cols<decltype(r)::value><<<(Ny + TZ - 1) / TZ, 256, cols_smem(), stream>>>(buf, twx, px, Ny, TZ, k, xy);
+        });
+        with_radix(py, [&](auto r) {
+            k2d_rows<decltype(r)::value><<<rows_grid, 256, rows_smem(), stream>>>(buf, eps, twy, py, G, nlines, +1, xy, rows_nbuf);
+        });
         launches += 4;
         M2_CUDA(cudaGetLastError());
         return M3D_OK;
@@ -341,17 +350,16 @@ int m3d2d_create(int Nx, int Ny, m3d_solver2d** out) {
     cudaMemcpy(h->twy, ty.data(), Ny * sizeof(double2), cudaMemcpyHostToDevice);
     cudaMemset(h->eps, 0, f);
     cudaMemset(h->sig, 0, f);
-// one limit per kernel for every handle (a per-handle value would lower it
+    // one limit per kernel for every handle (a per-handle value would lower it
     // under a larger handle made earlier): the device maximum
-    for (const void* k : {(const void*)k2d_rows, (const void*)k2d_cols}) {
-        cudaFuncAttributes a;
-        if (cudaFuncGetAttributes(&a, k) == cudaSuccess)
-            cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024 - (int)a.sharedSizeBytes);
-    }
+    with_radix(h->py, [&](auto r) { allow_smem(k2d_rows<decltype(r)::value>); });
+    with_radix(h->px, [&](auto r) { allow_smem(k2d_cols<decltype(r)::value>); });
     {
         int per_sm = 0, sms = 0, dev = 0;
         cudaGetDevice(&dev);
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k2d_rows, 256, h->rows_smem());
+        with_radix(h->py, [&](auto r) {
+            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k2d_rows<decltype(r)::value>, 256, h->rows_smem());
+        });
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
         const int tiles = (3 * Nx + h->G - 1) / h->G;
         h->rows_grid = std::max(1, std::min(tiles, std::max(1, per_sm) * std::max(1, sms)));
