@@ -605,11 +605,12 @@ enum Policy {
 
 // tot[s] = sum over the nblk block partials of sum s, in a fixed order (every
 // thread strides the same blocks, then a fixed tree) -> bit-reproducible.
-// Called by all threads of a block whose size is a power of two; the first
-// min(blockDim.x, 256) threads take part (red holds 256 doubles).
+// Called by all threads of a block of at least 32; the largest power of two of
+// them up to 256 take part (red holds 256 doubles).
 __device__ __forceinline__ void sum_partials(const double* partials, int NS, int nblk, int b, double* red,
                                              double* tot) {
-    const int nt = blockDim.x < 256 ? (int)blockDim.x : 256;
+    int nt = 256;
+    while (nt > (int)blockDim.x) nt >>= 1;
     for (int s = 0; s < NS; ++s) {
         const double* p = partials + ((long long)b * NS + s) * nblk;
         if (threadIdx.x < nt) {
@@ -659,7 +660,10 @@ struct FinLinear {
     __device__ __forceinline__ void run(Ctl* ctl, const double* partials, int NS, int nblk, int b, double* red,
                                         double* tot) const {
         sum_partials(partials, NS, nblk, b, red, tot);
-        if (threadIdx.x == 0) policy_linear(ctl[b], tot, policy, V, outer, b);
+        if (threadIdx.x == 0) {
+            if (NS < 2) tot[1] = 0;  // the residual policies use tot[0] only
+            policy_linear(ctl[b], tot, policy, V, outer, b);
+        }
     }
 };
 

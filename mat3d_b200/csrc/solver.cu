@@ -29,6 +29,7 @@
 #include "passes_slab.cuh"
 #include "fft_plan.hpp"
 #include "generic_launch.cuh"
+#include "plane_launch.cuh"
 
 #include <cudaTypedefs.h>
 
@@ -317,6 +318,8 @@ struct m3d_solver {
     // each warp)
     bool use_xcp = true;
     template <typename T> bool slab_ok() const;
+    template <typename T, int CC> bool plane_ok() const;
+    template <typename T, int CC> bool two_pass_ok() const { return plane_ok<T, CC>() || slab_ok<T>(); }
     template <typename T, int CC, bool MIX, class Fin>
     int pass_slab(Ctl* ctl, T* x, const float* r, typename Cx<T>::t* sp, Fin fin);
     template <typename T, int CC>
@@ -884,8 +887,25 @@ bool m3d_solver::slab_ok() const {
     return ok;
 }
 
+// Elastic operators couple the six components: the kz-plane pass and the z-mid
+// pass (passes_plane.cuh) where the length has a plane kernel.
+template <typename T, int CC>
+bool m3d_solver::plane_ok() const {
+    return CC == 6 && kind == M3D_KIND_MECH && use_fast && use_slab && Nx == Ny && Ny == Nz && plane_size<T>(Nz);
+}
+
 template <typename T, int CC, bool MIX, class Fin>
 int m3d_solver::pass_slab(Ctl* ctl, T* x, const float* r, typename Cx<T>::t* sp, Fin fin) {
+    if constexpr (CC == 6) {
+        if (plane_ok<T, CC>()) {
+            MidEMArgs<T> op = tab(MidEMArgs<T>{d_phase, x, r, g.V, dm(off_P), dm(off_A), nph_max()});
+            FinLinear fl{};
+            if constexpr (MIX) fl = fin;
+            M3D_CUDA(zmid_pass<T>(Nz, gridB(), MIX, stream, g, tw<T>(2), sp, op, ctl, d_part, fl));
+            st.kernel_launches += 1;
+            return M3D_OK;
+        }
+    }
     SlabOps<T> ops{CC, d_phase, x, r, dm(off_P), dm(off_A), dm(off_Os), nph_max(), entries_per_rve(), mstride};
     bool done = false;
     with_fast_n(Nz, [&](auto nc) {
@@ -920,7 +940,15 @@ int m3d_solver::launch_em_slab(Ctl* ctl, T* x, const float* r, typename Cx<T>::t
     prof_pass(0);
     prof_pass(1);
     prof_pass(2);
-    pass_x<T, CC>(green<T, CC>(zero_k0), ctl, sp);
+    bool plane = false;
+    if constexpr (CC == 6) {
+        plane = plane_ok<T, CC>();
+        if (plane) {
+            M3D_CUDA(plane_pass<T>(Nz, gridB(), stream, g, tw<T>(2), sp, green<T, CC>(zero_k0), ctl));
+            st.kernel_launches += 1;
+        }
+    }
+    if (!plane) pass_x<T, CC>(green<T, CC>(zero_k0), ctl, sp);
     prof_pass(3);
     prof_pass(4);
     const int rc = pass_slab<T, CC, true>(ctl, x, r, sp, FinLinear{policy, (double)g.V, outer, d_counter});
@@ -949,7 +977,7 @@ int m3d_solver::run_linear(double tol_field, double tol_eq, int criterion, int m
     C2* sp = (C2*)d_spec;
     const int chunk = kChunk;
     int before = 0;
-    const bool slab = criterion == M3D_CRIT_RESIDUAL && slab_ok<T>();
+    const bool slab = criterion == M3D_CRIT_RESIDUAL && two_pass_ok<T, CC>();
     st.passes_per_sweep = slab ? 2 : 5;
     if (slab) {
         rc = pass_slab<T, CC, false>(d_ctl, x, nullptr, sp, FinNone{});
@@ -1010,7 +1038,7 @@ int m3d_solver::run_refine(double tol_field, int max_iter) {
     long long n64 = 0, n32 = 0;
     bool first = true;
     const int chunk = 8;
-    const bool slab = slab_ok<float>();
+    const bool slab = two_pass_ok<float, CC>();
     st.passes_per_sweep = slab ? 2 : 5;
     std::vector<long long> in32((size_t)B, 0);  // FP32 sweeps per entry
     for (;;) {
@@ -1261,7 +1289,7 @@ int m3d_solver::run_linear_graph(double tol_field, double tol_eq, int criterion,
     k_fill_load<T><<<dim3(256, B * CC), 256, 0, stream>>>(x, d_ctl, CC, g.V);
     M3D_CUDA(cudaMemsetAsync(d_trips, 0, 8 * sizeof(int), stream));
     const bool resid = (criterion == M3D_CRIT_RESIDUAL);
-    const bool slab = resid && slab_ok<T>();
+    const bool slab = resid && two_pass_ok<T, CC>();
     st.passes_per_sweep = slab ? 2 : 5;
     if (slab) {
         rc = pass_slab<T, CC, false>(d_ctl, x, nullptr, sp, FinNone{});
@@ -1358,7 +1386,7 @@ int m3d_solver::run_refine_graph(double tol_field, int max_iter) {
     M3D_CUDA(cudaMemsetAsync(d_delta, 0, dbytes, stream));
     M3D_CUDA(cudaMemsetAsync(d_ctl_in, 0, (size_t)B * sizeof(Ctl), stream));
     M3D_CUDA(cudaMemsetAsync(d_trips, 0, 8 * sizeof(int), stream));
-    const bool slab = slab_ok<float>();
+    const bool slab = two_pass_ok<float, CC>();
     st.passes_per_sweep = slab ? 2 : 5;
     const size_t sbytes32 = (size_t)B * CC * g.NL * g.Hzp * sizeof(float2);
     GraphSlot& gs = gslot[2];
@@ -2259,7 +2287,7 @@ int m3d_solver::tune_time(int sweeps, float* ms) {
     cudaEvent_t e0, e1;
     M3D_CUDA(cudaEventCreate(&e0));
     M3D_CUDA(cudaEventCreate(&e1));
-    const bool slab = slab_ok<T>();
+    const bool slab = two_pass_ok<T, CC>();
     auto sweep = [&]() {
         return slab ? launch_em_slab<T, CC>(d_ctl, x, r, sp, 0, POL_RESIDUAL, nullptr)
                     : launch_em<T, CC>(d_ctl, x, r, sp, 0, POL_RESIDUAL, nullptr);
@@ -2291,7 +2319,8 @@ int m3d_solver::autotune(int sweeps, m3d_tune* out) {
         cand.push_back(m3d_tune{1, 1, G0, Y0, X0, 0, 0, 0, 0});
         const bool f1 = use_fast, s1 = use_slab;
         use_fast = use_slab = true;
-        const bool slab_possible = fp64 ? slab_ok<double>() : slab_ok<float>();
+        const bool slab_possible = fp64 ? (C == 6 ? two_pass_ok<double, 6>() : two_pass_ok<double, 3>())
+                                        : (C == 6 ? two_pass_ok<float, 6>() : two_pass_ok<float, 3>());
         use_fast = f1;
         use_slab = s1;
         if (slab_possible) cand.push_back(m3d_tune{1, 0, G0, Y0, X0, 0, 0, 1, 0});
