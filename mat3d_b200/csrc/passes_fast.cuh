@@ -274,15 +274,20 @@ constexpr size_t xturn_cp_smem() {
            (size_t)32 * (NSUM > 0 ? NSUM : 1) * sizeof(double);
 }
 
-// CTAs per SM of the six-component FP32 kernel at N = 96: three (a cap of
-// 112 registers instead of 152, 140 bytes of spill; the batch workload's
-// 96^3 group's x turnaround 157 -> 142 ms on one box, bitwise the same).  At
-// 64^3 the same cap timed equal; FP64 and N = 256 spill up to 1 KB under it.
-#ifndef M3D_XCP_MINB
-#define M3D_XCP_MINB 3
-#endif
+// CTAs per SM of the component-parallel x turnaround (its register cap).  Six
+// warps of more than 170 registers run one CTA per SM: uncapped the long FP64
+// lines take 176-220 and FP32 256 points 185.  Measured per launch, six
+// components: FP64 256^3 887 us uncapped, 625 at two CTAs (no spill), 599 at
+// three (116 bytes); FP32 256^3 531, 398, 425 (200 bytes).  FP32 96^3 three
+// (140 bytes of spill; 157 -> 142 ms of a batch group's x turnaround), FP64 96^3
+// two.  Three warps of 178-236 registers: four CTAs of 168.
+template <typename T, int N, int C> struct XcpMinB {
+    static constexpr int value = C == 3 ? ((N == 256 || (sizeof(T) == 8 && N >= 96)) ? 4 : 1)
+                                        : (sizeof(T) == 8 && N >= 128) ? 3
+                                        : N == 256 ? 2 : N == 96 ? (sizeof(T) == 4 ? 3 : 2) : 1;
+};
 template <typename T, int N, int C, class Spec>
-__global__ void __launch_bounds__(32 * C, (C == 6 && sizeof(T) == 4 && N == 96) ? M3D_XCP_MINB : 1) k_xturn_cp(GridDims g, const typename Cx<T>::t* __restrict__ twx,
+__global__ void __launch_bounds__(32 * C, XcpMinB<T, N, C>::value) k_xturn_cp(GridDims g, const typename Cx<T>::t* __restrict__ twx,
                                                      typename Cx<T>::t* __restrict__ spec, Spec op,
                                                      const Ctl* __restrict__ ctl, double* partials) {
     typedef typename Cx<T>::t C2;
