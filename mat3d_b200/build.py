@@ -23,7 +23,7 @@ NVCC_FLAGS = [
 ]
 
 SOURCES = [os.path.join(CSRC, "solver.cu"), os.path.join(CSRC, "generic_r31.cu"),
-           os.path.join(CSRC, "generic_r13.cu"), os.path.join(CSRC, "plane.cu"), os.path.join(CSRC, "noalloc.cu"), os.path.join(CSRC, "compat.cpp"),
+           os.path.join(CSRC, "generic_r13.cu"), os.path.join(CSRC, "plane.cu"), os.path.join(CSRC, "zmid.cu"), os.path.join(CSRC, "noalloc.cu"), os.path.join(CSRC, "compat.cpp"),
            os.path.join(CSRC, "batch.cpp"), os.path.join(CSRC, "serve.cpp"),
            os.path.join(CSRC, "solver2d.cu"), os.path.join(CSRC, "rec.cu"), os.path.join(CSRC, "rec_compat.cpp")]
 DEPS = SOURCES + [os.path.join(CSRC, f) for f in os.listdir(CSRC)] + [

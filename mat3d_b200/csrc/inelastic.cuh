@@ -41,9 +41,27 @@ __device__ __forceinline__ double vonmises(const double (&s)[6], double (&sd)[6]
 // the rest of the update.
 __device__ __forceinline__ double hpow(double x, double n) { return n == 1.0 ? x : (n == 0.0 ? 1.0 : pow(x, n)); }
 
-// J2 return map (elastoPlastic, :640-691).  Returns dp (0 when elastic), sets
-// sig, phi.  NR on the plastic multiplier from 0 with the reference's absolute
-// tolerance 1e-5 on the yield function, capped at 200 steps (*nr_fail set).
+// Plastic multiplier of the J2 return map (elastoPlastic, :640-691) for the
+// trial stress's von Mises value: 0 when elastic, else Newton-Raphson from 0
+// with the reference's absolute tolerance 1e-5 on the yield function, capped at
+// 200 steps (*nr_fail set).
+__device__ __forceinline__ double j2_multiplier(double seff, double ep, double mu, double Sy, double H, double n,
+                                                int* nr_fail) {
+    if (!(seff - Sy - H * hpow(ep, n) > 0)) return 0.0;
+    double x = 0, xo = 0;
+    int it = 0;
+    for (;;) {
+        x = xo - (seff - 3 * mu * xo - Sy - H * hpow(ep + xo, n)) / (-3 * mu - H * n * hpow(ep + xo, n - 1));
+        xo = x;
+        const double res = seff - 3 * mu * x - Sy - H * hpow(ep + x, n);
+        if (!(x == x)) { *nr_fail = 1; break; }
+        if (fabs(res) < 1e-5) break;
+        if (++it >= 200) { *nr_fail = 1; break; }
+    }
+    return x;
+}
+
+// J2 return map.  Returns dp (0 when elastic), sets sig, phi.
 __device__ __forceinline__ double j2_update(const PhaseMech& P, const double (&eps)[6], const double (&eps_old)[6],
                                             const double (&sig_old)[6], double ep, double (&sig)[6], double& phi,
                                             int* nr_fail) {
@@ -61,17 +79,7 @@ __device__ __forceinline__ double j2_update(const PhaseMech& P, const double (&e
     const double seff = vonmises(sig, sd);
     phi = seff - P.Sy - P.H * hpow(ep, P.n);
     if (!(phi > 0)) return 0.0;
-    double x = 0, xo = 0;
-    int it = 0;
-    for (;;) {
-        x = xo - (seff - 3 * P.mu * xo - P.Sy - P.H * hpow(ep + xo, P.n)) /
-                     (-3 * P.mu - P.H * P.n * hpow(ep + xo, P.n - 1));
-        xo = x;
-        const double res = seff - 3 * P.mu * x - P.Sy - P.H * hpow(ep + x, P.n);
-        if (!(x == x)) { *nr_fail = 1; break; }
-        if (fabs(res) < 1e-5) break;
-        if (++it >= 200) { *nr_fail = 1; break; }
-    }
+    const double x = j2_multiplier(seff, ep, P.mu, P.Sy, P.H, P.n, nr_fail);
     // sig -= (1.5 x / seff) C sd
     const double f = 1.5 * x / seff;
 #pragma unroll
@@ -281,11 +289,13 @@ struct EpiBasic {
     __device__ __forceinline__ void apply(int b, long long v, T (&xc)[6], double* acc) const { c.apply(b, v, xc, acc); }
 };
 
-// standalone constitutive pass (increment start), same sums
+// standalone constitutive pass (increment start), same sums; at the end of an
+// increment whose sweeps do not store the stress (mid_ops.cuh) it writes the
+// stress of the converged strain (all = 1: entries that are done too)
 template <typename T>
-__global__ void k_constitutive(EpiConstitutive<T> epi, const Ctl* ctl, double* partials) {
+__global__ void k_constitutive(EpiConstitutive<T> epi, const Ctl* ctl, double* partials, int all) {
     const int b = blockIdx.y;
-    if (ctl[b].done) return;
+    if (!all && ctl[b].done) return;
     extern __shared__ __align__(16) char smem_raw[];
     double* red = (double*)smem_raw;
     epi.bind(b);

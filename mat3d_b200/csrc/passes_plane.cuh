@@ -42,7 +42,8 @@
 #pragma once
 #include <cooperative_groups.h>
 
-#include "passes_fast.cuh"
+#include "line_at.cuh"
+#include "mid_ops.cuh"
 
 namespace m3d {
 
@@ -74,50 +75,6 @@ M3D_PLANE(double, 64, 1, 128, 3)
 // Green operator needs to know.
 template <typename T> __device__ __forceinline__ int plane_swz(int row) {
     return sizeof(T) == 4 ? (((row & 1) << 3) | ((row & 2) << 1)) : ((row & 1) << 2);
-}
-
-// line_fwd / line_inv (fft_reg.cuh) with the exchange through at(k1, u):
-// element k1*T + u of the line's own storage
-template <typename C2, int E, int T, class At>
-__device__ __forceinline__ void line_fwd_at(C2 (&v)[E], int t, const C2* tw, At at) {
-    constexpr int N = E * T, Q = E / T;
-    dft_reg<C2, E, N>(v, tw, -1);
-#pragma unroll
-    for (int k1 = 1; k1 < E; ++k1) v[k1] = cmul(v[k1], twid(tw, t * k1, -1));
-    __syncwarp();  // every lane of the line has read its inputs
-#pragma unroll
-    for (int k1 = 0; k1 < E; ++k1) *at(k1, t ^ (k1 / Q)) = v[k1];
-    __syncwarp();
-#pragma unroll
-    for (int q = 0; q < Q; ++q) {
-        C2 u[T];
-#pragma unroll
-        for (int t2 = 0; t2 < T; ++t2) u[t2] = *at(t * Q + q, t2 ^ t);
-        dft_reg<C2, T, N>(u, tw, -1);
-#pragma unroll
-        for (int k2 = 0; k2 < T; ++k2) v[q * T + k2] = u[k2];
-    }
-    __syncwarp();
-}
-template <typename C2, int E, int T, class At>
-__device__ __forceinline__ void line_inv_at(C2 (&v)[E], int t, const C2* tw, At at) {
-    constexpr int N = E * T, Q = E / T;
-    __syncwarp();
-#pragma unroll
-    for (int q = 0; q < Q; ++q) {
-        C2 u[T];
-#pragma unroll
-        for (int k2 = 0; k2 < T; ++k2) u[k2] = v[q * T + k2];
-        dft_reg<C2, T, N>(u, tw, +1);
-        const int k1 = t * Q + q;
-#pragma unroll
-        for (int t2 = 0; t2 < T; ++t2) *at(k1, t2 ^ t) = (t2 == 0) ? u[t2] : cmul(u[t2], twid(tw, t2 * k1, +1));
-    }
-    __syncwarp();
-#pragma unroll
-    for (int k1 = 0; k1 < E; ++k1) v[k1] = *at(k1, t ^ (k1 / Q));
-    __syncwarp();
-    dft_reg<C2, E, N>(v, tw, +1);
 }
 
 // -G(xi) of one mode as SpecGreen, with one reciprocal for both schemes
@@ -282,116 +239,6 @@ __global__ void __launch_bounds__(PlaneGeom<T, N>::NT, PlaneGeom<T, N>::MINB)
 // ---------------------------------------------------------------------------
 // z-mid pass
 // ---------------------------------------------------------------------------
-// EM update and polarization of isotropic phases: A d = a_l tr(d) I + a_s d
-// and P x likewise, two constants per phase and table instead of 36 (every
-// phase of the mechanical solver is isotropic, so C, S, C - C0, S - S0 and
-// 2 (C + C0)^-1 C0 are).  Sums: [0] sum w d^2.
-template <typename T>
-struct MidEMArgs {
-    const uint8_t* phase;
-    T* x;
-    const float* r;       // defect forcing of the correction solve, may be null
-    long long V;
-    const double* P;      // [nph][6][6]
-    const double* A;
-    int nph;
-    int lc = 0;           // batch entries per RVE (0: one RVE shared by all)
-    long long mstride = 0;
-};
-// W consecutive voxels per item: with two in FP32 the global accesses are 8
-// bytes a lane and a tile access a whole 16-byte pair of complex elements
-template <typename T, int W_>
-struct MidEM {
-    static constexpr int NSUM = 1, W = W_;
-    typedef MidEMArgs<T> Args;
-    Args a;
-    long long V;
-    struct Coef { T al, as, pl, ps; };
-    const Coef* sm = nullptr;
-    const uint8_t* phb = nullptr;
-    T* xb = nullptr;
-    const float* rb = nullptr;
-    __device__ __forceinline__ void bind(int b) {
-        V = a.V;
-        phb = a.phase + (a.lc ? (long long)(b / a.lc) * V : 0);
-        xb = a.x + (long long)b * 6 * V;
-        rb = a.r ? a.r + (long long)b * 6 * V : nullptr;
-    }
-    __device__ __forceinline__ void load_smem(char* s, int b) {
-        Coef* c = (Coef*)s;
-        const long long o = a.lc ? (long long)(b / a.lc) * a.mstride : 0;
-        for (int i = threadIdx.x; i < a.nph; i += blockDim.x)
-            c[i] = Coef{(T)a.A[o + i * 36 + 1], (T)a.A[o + i * 36 + 21], (T)a.P[o + i * 36 + 1], (T)a.P[o + i * 36 + 21]};
-        sm = c;
-    }
-    struct In {
-        int p[W];
-        T x[6][W];
-        float r[6][W];
-    };
-    template <bool MIX> __device__ __forceinline__ void load(long long v, In& q) const {
-        if constexpr (W == 2) {
-            const uchar2 u = *reinterpret_cast<const uchar2*>(phb + v);
-            q.p[0] = u.x;
-            q.p[1] = u.y;
-        } else {
-            q.p[0] = phb[v];
-        }
-#pragma unroll
-        for (int c = 0; c < 6; ++c) {
-            if constexpr (W == 2) {
-                const float2 u = *reinterpret_cast<const float2*>(xb + c * V + v);
-                q.x[c][0] = u.x;
-                q.x[c][1] = u.y;
-            } else {
-                q.x[c][0] = xb[c * V + v];
-            }
-            if constexpr (MIX) {
-                if constexpr (W == 2) {
-                    const float2 u = rb ? *reinterpret_cast<const float2*>(rb + c * V + v) : make_float2(0.f, 0.f);
-                    q.r[c][0] = u.x;
-                    q.r[c][1] = u.y;
-                } else {
-                    q.r[c][0] = rb ? rb[c * V + v] : 0.f;
-                }
-            }
-        }
-    }
-    // f: in the transform's values x_c of W voxels, out their polarization
-    template <bool MIX> __device__ __forceinline__ void apply(const In& q, long long v, T (&f)[6][W], double* acc) const {
-        T xn[6][W];
-#pragma unroll
-        for (int w = 0; w < W; ++w) {
-            const Coef k = sm[q.p[w]];
-            if constexpr (MIX) {
-                T d[6];
-#pragma unroll
-                for (int c = 0; c < 6; ++c) d[c] = (f[c][w] + (T)q.r[c][w]) - q.x[c][w];
-                double rs = 0;
-#pragma unroll
-                for (int c = 0; c < 6; ++c) rs += (c < 3 ? 1.0 : 2.0) * (double)d[c] * (double)d[c];
-                acc[0] += rs;
-                const T tr = k.al * (d[0] + d[1] + d[2]);
-#pragma unroll
-                for (int c = 0; c < 6; ++c) xn[c][w] = q.x[c][w] + (c < 3 ? k.as * d[c] + tr : k.as * d[c]);
-            } else {
-#pragma unroll
-                for (int c = 0; c < 6; ++c) xn[c][w] = q.x[c][w];
-            }
-            const T tp = k.pl * (xn[0][w] + xn[1][w] + xn[2][w]);
-#pragma unroll
-            for (int c = 0; c < 6; ++c) f[c][w] = c < 3 ? k.ps * xn[c][w] + tp : k.ps * xn[c][w];
-        }
-        if constexpr (MIX) {
-#pragma unroll
-            for (int c = 0; c < 6; ++c) {
-                if constexpr (W == 2) *reinterpret_cast<float2*>(xb + c * V + v) = make_float2(xn[c][0], xn[c][1]);
-                else xb[c * V + v] = xn[c][0];
-            }
-        }
-    }
-};
-
 // G lines (consecutive y) of six components: 3 G complex lines, each the pair
 // (2p, 2p+1) of a voxel line, row p*G + gi of the tile; a warp owns eight lines
 // of one pair, so it loads, transforms, splits and stores its rows without a
@@ -422,21 +269,6 @@ template <typename T, int N> struct ZMidGeom {
         return (size_t)N * 2 * sizeof(T) + (size_t)LINES * ROW * 2 * sizeof(T) + 64 * sizeof(double) + kMaxPhases * 4 * sizeof(T);
     }
 };
-
-__device__ __forceinline__ void cp_async_c(float2* d, const float2* s) { cp_async(d, s, 8, 8); }
-__device__ __forceinline__ void cp_async_c(double2* d, const double2* s) { cp_async(d, s, 16, 16); }
-
-// W consecutive complex elements of a tile row
-__device__ __forceinline__ void tile_get(const float2* p, float2 (&u)[2]) {
-    const float4 v = *reinterpret_cast<const float4*>(p);
-    u[0] = make_float2(v.x, v.y);
-    u[1] = make_float2(v.z, v.w);
-}
-__device__ __forceinline__ void tile_put(float2* p, const float2 (&u)[2]) {
-    *reinterpret_cast<float4*>(p) = make_float4(u[0].x, u[0].y, u[1].x, u[1].y);
-}
-template <typename C2> __device__ __forceinline__ void tile_get(const C2* p, C2 (&u)[1]) { u[0] = *p; }
-template <typename C2> __device__ __forceinline__ void tile_put(C2* p, const C2 (&u)[1]) { *p = u[0]; }
 
 template <typename T, int N, class Op, bool MIX, class Fin>
 __global__ void __launch_bounds__(ZMidGeom<T, N>::NT, ZMidGeom<T, N>::MINB)

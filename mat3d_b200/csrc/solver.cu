@@ -30,6 +30,7 @@
 #include "fft_plan.hpp"
 #include "generic_launch.cuh"
 #include "plane_launch.cuh"
+#include "zmid_launch.cuh"
 
 #include <cudaTypedefs.h>
 

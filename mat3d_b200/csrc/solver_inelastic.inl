@@ -180,6 +180,12 @@ int m3d_solver::run_inelastic(double tol_field, double tol_eq, int nInc, int cri
     // stress increment (J2 keeps the previous step's stress)
     if (sizeof(T) == 4 && criterion == M3D_CRIT_RESIDUAL && sig_old) pro.sig_old = sig_old;
     SpecBasic<T> spec{green<T, 6>(0), SpecEqVar<T, 6>{g}};
+    // fused z pass (z inverse, update, next z forward) where Nz has one; the
+    // stress then stays in registers and is written at the end of an increment
+    const bool mid = use_fast && use_slab && zmid_rows_ok<T>(Nz, g.NL);
+    const MidJ2Args margs{d_phase, eps, eps_old, sig_old, ep, dmg, V, in.d_ph, nph, pro.sig_old ? 1 : 0, in.d_nrfail};
+    // the convergence sums of the stress spectrum are the reference rule's alone
+    const bool check = criterion == M3D_CRIT_REFERENCE;
     const size_t phb = (size_t)nph * sizeof(PhaseMech) + 64;
     const int cblk = 592;
     const size_t csmem = 32 * 32 * 8 + phb;
@@ -198,27 +204,37 @@ int m3d_solver::run_inelastic(double tol_field, double tol_eq, int nInc, int cri
             h_ctl[b].aux[AUX_DESUM] = s * (inc + 1);
         }
         M3D_CUDA(cudaMemcpyAsync(d_ctl, h_ctl, B * sizeof(Ctl), cudaMemcpyHostToDevice, stream));
-        k_constitutive<T><<<dim3(cblk, B), 256, csmem, stream>>>(cons, d_ctl, d_part);
+        k_constitutive<T><<<dim3(cblk, B), 256, csmem, stream>>>(cons, d_ctl, d_part, 0);
         k_finalize_j2<<<B, 256, 0, stream>>>(d_ctl, d_part, 13, cblk, POLJ2_START, (double)V, in.d_S0);
         st.kernel_launches += 2;
         int before = 0;
+        if (mid) pass_zfwd<T, 6>(pro, d_ctl, sp);
         for (;;) {
             for (int k = 0; k < chunk; ++k) {
                 prof_mark(k);
                 prof_pass(0);
-                pass_zfwd<T, 6>(pro, d_ctl, sp);
+                if (!mid) pass_zfwd<T, 6>(pro, d_ctl, sp);
                 prof_pass(1);
                 pass_y<T>(-1, 6, d_ctl, sp);
                 prof_pass(2);
-                const int xblk = pass_x<T, 6>(spec, d_ctl, sp);
-                if (criterion == M3D_CRIT_REFERENCE) {
+                if (check) {
+                    const int xblk = pass_x<T, 6>(spec, d_ctl, sp);
                     k_finalize_j2<<<B, 256, 0, stream>>>(d_ctl, d_part, 2, xblk, POLJ2_CHECK, (double)V, in.d_S0);
                     st.kernel_launches += 1;
+                } else {
+                    pass_x<T, 6>(spec.green, d_ctl, sp);
                 }
                 prof_pass(3);
                 pass_y<T>(+1, 6, d_ctl, sp);
                 prof_pass(4);
-                pass_zinv<T, 6>(epi, d_ctl, sp, FinJ2{POLJ2_SWEEP, (double)V, in.d_S0, d_counter});
+                const FinJ2 fin{POLJ2_SWEEP, (double)V, in.d_S0, d_counter};
+                if (mid) {
+                    M3D_CUDA(zmid_rows_inelastic<T>(Nz, behav == M3D_BEHAV_J2, B, stream, g, tw<T>(2), sp, margs, d_ctl,
+                                                    d_part, fin));
+                    st.kernel_launches += 1;
+                } else {
+                    pass_zinv<T, 6>(epi, d_ctl, sp, fin);
+                }
                 prof_pass(5);
             }
             M3D_CUDA(cudaGetLastError());
@@ -230,6 +246,10 @@ int m3d_solver::run_inelastic(double tol_field, double tol_eq, int nInc, int cri
             bool all = true;
             for (int b = 0; b < B; ++b) all = all && h_ctl[b].done;
             if (all) break;
+        }
+        if (mid) {
+            k_constitutive<T><<<dim3(cblk, B), 256, csmem, stream>>>(cons, d_ctl, d_part, 1);
+            st.kernel_launches += 1;
         }
         for (int b = 0; b < B; ++b) {
             total += h_ctl[b].iters;

@@ -1,0 +1,59 @@
+// zmid.cu -- the fused z pass on the row layout: kernels and launches.
+#include <algorithm>
+
+#include "generic_launch.cuh"  // allow_smem
+#include "zmid_launch.cuh"
+
+namespace m3d {
+
+namespace {
+template <int NN> struct IntC { static constexpr int value = NN; };
+template <class F> void with_n(int n, F&& f) {
+    switch (n) {
+        case 32: f(IntC<32>{}); break;
+        case 48: f(IntC<48>{}); break;
+        case 64: f(IntC<64>{}); break;
+        case 96: f(IntC<96>{}); break;
+        case 128: f(IntC<128>{}); break;
+        case 256: f(IntC<256>{}); break;
+        default: break;
+    }
+}
+template <typename T, int NN, int C, class Op, class Fin>
+cudaError_t go(int entries, cudaStream_t st, const GridDims& g, const typename Cx<T>::t* tw, typename Cx<T>::t* sp,
+               const typename Op::Args& op, Ctl* ctl, double* part, const Fin& fin) {
+    typedef ZRowsGeom<T, NN, C> Z;
+    auto kern = k_zmid_rows<T, NN, C, Op, Fin>;
+    allow_smem(kern);
+    kern<<<dim3((unsigned)std::min<long long>(g.NL / Z::G, kZRowsGrid), entries), Z::NT, Z::template smem<Op>(op.nph), st>>>(g, tw, sp, op, ctl, part, fin);
+    return cudaGetLastError();
+}
+}  // namespace
+
+template <typename T>
+bool zmid_rows_ok(int N, long long NL) {
+    bool ok = false;
+    with_n(N, [&](auto nc) { ok = NL % ZRowsGeom<T, decltype(nc)::value, 6>::G == 0; });
+    return ok;
+}
+template bool zmid_rows_ok<float>(int, long long);
+template bool zmid_rows_ok<double>(int, long long);
+
+template <typename T>
+cudaError_t zmid_rows_inelastic(int N, bool j2, int entries, cudaStream_t st, const GridDims& g,
+                                const typename Cx<T>::t* tw, typename Cx<T>::t* sp, const MidJ2Args& op, Ctl* ctl,
+                                double* part, const FinJ2& fin) {
+    cudaError_t e = cudaErrorInvalidValue;
+    with_n(N, [&](auto nc) {
+        constexpr int NN = decltype(nc)::value;
+        e = j2 ? go<T, NN, 6, MidJ2<T, true>, FinJ2>(entries, st, g, tw, sp, op, ctl, part, fin)
+               : go<T, NN, 6, MidJ2<T, false>, FinJ2>(entries, st, g, tw, sp, op, ctl, part, fin);
+    });
+    return e;
+}
+template cudaError_t zmid_rows_inelastic<float>(int, bool, int, cudaStream_t, const GridDims&, const float2*, float2*,
+                                                const MidJ2Args&, Ctl*, double*, const FinJ2&);
+template cudaError_t zmid_rows_inelastic<double>(int, bool, int, cudaStream_t, const GridDims&, const double2*, double2*,
+                                                 const MidJ2Args&, Ctl*, double*, const FinJ2&);
+
+}  // namespace m3d
