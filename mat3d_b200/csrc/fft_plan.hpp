@@ -9,37 +9,69 @@
 
 namespace m3d {
 
-// radix schedule: odd primes up to kMaxGenericRadix, largest first (the
-// first stage needs no twiddle multiplications, so the costliest butterfly
-// goes there), then 8, 4, 2; false if a factor is larger
-// (fuse9: two factors 3 become one radix-9 stage -- one Stockham stage and
-// barrier fewer -- for callers whose kernels compile the 9-point butterfly).
-// Any order of the factors is a valid Stockham schedule; `order` picks one
-// for the autotuner: 0 the above, 1 odd factors smallest first, 2 the
-// power-of-two stages first, 3 the power of two as radix-4 stages (and one 2).
+// The radices of the factors 2, 3 and 5 with a register DFT; the primes above
+// come one per stage.
+constexpr int kRadices[] = {16, 15, 12, 10, 9, 8, 6, 5, 4, 3, 2};
+// The fewest of kRadices (largest first) whose product is m, among those the
+// smallest sum.
+inline void fewest_radices(int m, std::vector<int>& cur, std::vector<int>& best, bool& have) {
+    auto sum = [](const std::vector<int>& v) {
+        int t = 0;
+        for (int r : v) t += r;
+        return t;
+    };
+    if (m == 1) {
+        if (!have || cur.size() < best.size() || (cur.size() == best.size() && sum(cur) < sum(best))) best = cur;
+        have = true;
+        return;
+    }
+    if (have && cur.size() + 1 > best.size()) return;
+    for (int r : kRadices)
+        if (m % r == 0 && (cur.empty() || r <= cur.back())) {
+            cur.push_back(r);
+            fewest_radices(m / r, cur, best, have);
+            cur.pop_back();
+        }
+}
+
+// radix schedule of a length; false if a prime factor is above 31.  Any order
+// and grouping of the factors is a valid Stockham schedule; `order` picks one
+// for the autotuner: 0 as few stages as possible, the primes above 5 first
+// (the first stage needs no twiddle multiplications, so the costliest
+// butterfly goes there), then by radix; 1 one factor per stage, odd factors
+// smallest first, then 8s, 4, 2; 2 the power-of-two stages first; 3 odd factors
+// largest first, the power of two as radix-4 stages (and one 2).
 constexpr int kPlanOrders = 4;
-inline bool make_plan(int n, LinePlan& p, bool fuse9 = false, int order = 0) {
+inline bool make_plan(int n, LinePlan& p, int order = 0) {
     std::vector<int> f, odd;
     int m = n;
     int p2 = 0;
     while (m % 2 == 0) { ++p2; m /= 2; }
-    if (fuse9)
-        while (m % 9 == 0) { odd.push_back(9); m /= 9; }
     for (int q = 3; q <= m; q += 2)
-        while (m % q == 0) { odd.push_back(q); m /= q; }
-    std::sort(odd.begin(), odd.end());
-    std::vector<int> pow2;
-    if (order == 3) {
-        for (; p2 >= 2; p2 -= 2) pow2.push_back(4);
+        while (m % q == 0) { odd.push_back(q); m /= q; }  // ascending
+    if (order == 0) {
+        int smooth = 1 << p2;
+        for (size_t i = odd.size(); i-- > 0;)
+            if (odd[i] > 5) f.push_back(odd[i]);
+            else smooth *= odd[i];
+        std::vector<int> cur, best;
+        bool have = false;
+        fewest_radices(smooth, cur, best, have);
+        f.insert(f.end(), best.begin(), best.end());
     } else {
-        for (; p2 >= 3; p2 -= 3) pow2.push_back(8);
-        if (p2 == 2) pow2.push_back(4);
+        std::vector<int> pow2;
+        if (order == 3) {
+            for (; p2 >= 2; p2 -= 2) pow2.push_back(4);
+        } else {
+            for (; p2 >= 3; p2 -= 3) pow2.push_back(8);
+            if (p2 == 2) pow2.push_back(4);
+        }
+        if (p2 == 1) pow2.push_back(2);
+        if (order == 2) f = pow2;
+        if (order == 1) f.insert(f.end(), odd.begin(), odd.end());
+        else f.insert(f.end(), odd.rbegin(), odd.rend());
+        if (order != 2) f.insert(f.end(), pow2.begin(), pow2.end());
     }
-    if (p2 == 1) pow2.push_back(2);
-    if (order == 2) f = pow2;
-    if (order == 1) f.insert(f.end(), odd.begin(), odd.end());
-    else f.insert(f.end(), odd.rbegin(), odd.rend());
-    if (order != 2) f.insert(f.end(), pow2.begin(), pow2.end());
     if (f.empty()) f.push_back(1);
     if ((int)f.size() > kMaxStages) return false;
     for (int r : f)
@@ -47,7 +79,17 @@ inline bool make_plan(int n, LinePlan& p, bool fuse9 = false, int order = 0) {
     p.n = n;
     p.nstages = (n == 1) ? 0 : (int)f.size();
     for (int i = 0; i < kMaxStages; ++i) p.radix[i] = i < (int)f.size() ? f[i] : 1;
+    finish_plan(p);
     return true;
+}
+
+// Threads of a CTA that transforms `lines` lines of plan p together: one per
+// butterfly of its widest stage, 64 to 256.
+inline int plan_threads(const LinePlan& p, int lines) {
+    int r = 1;
+    for (int s = 0; s < p.nstages; ++s) r = std::max(r, p.radix[s]);
+    const int b = lines * (p.n / r);
+    return std::max(64, std::min(256, (b + 31) / 32 * 32));
 }
 
 // tw[m] = exp(-2 pi i m / n), evaluated in long double

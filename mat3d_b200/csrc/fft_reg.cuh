@@ -18,47 +18,6 @@
 
 namespace m3d {
 
-// exp(-+2 pi i m / L) for L dividing 96, m known at compile time: the sub-DFT
-// twiddles inside the register DFTs.  As immediates they cost neither the
-// broadcast shared-memory loads nor the registers of table entries (a radix-24
-// DFT multiplies by 15 of them); thermal 128^3 refinement 11.44 -> 11.33 ms a
-// solve.  Not for the radix-32 DFT, whose y forward pass at FP32 256^3 went from
-// 102 to 155 us with them.  cos and sin of
-// 2 pi k / 96 in the first octant, mirrored into the others; the switches fold
-// away once the loops over m are unrolled.
-template <typename T>
-__device__ __forceinline__ void octant96(int k, T& c, T& s) {
-    switch (k) {
-        case 0: c = (T)1.0000000000000000000000; s = (T)0.0; break;
-        case 1: c = (T)0.9978589232386035067380; s = (T)0.0654031292301430668153; break;
-        case 2: c = (T)0.9914448613738104111445; s = (T)0.1305261922200515915484; break;
-        case 3: c = (T)0.9807852804032304491261; s = (T)0.1950903220161282678482; break;
-        case 4: c = (T)0.9659258262890682867497; s = (T)0.2588190451025207623488; break;
-        case 5: c = (T)0.9469301294951056642558; s = (T)0.3214394653031615807010; break;
-        case 6: c = (T)0.9238795325112867561281; s = (T)0.3826834323650897717284; break;
-        case 7: c = (T)0.8968727415326883038941; s = (T)0.4422886902190012819952; break;
-        case 8: c = (T)0.8660254037844386467637; s = (T)0.5000000000000000000000; break;
-        case 9: c = (T)0.8314696123025452370787; s = (T)0.5555702330196022247428; break;
-        case 10: c = (T)0.7933533402912351645797; s = (T)0.6087614290087206394160; break;
-        case 11: c = (T)0.7518398074789773964075; s = (T)0.6593458151000688684251; break;
-        default: c = (T)0.7071067811865475244008; s = (T)0.7071067811865475244008; break;
-    }
-}
-// a * exp(sign 2 pi i m / L)
-template <typename C2, int L>
-__device__ __forceinline__ C2 rot_const(C2 a, int m, int sign) {
-    typedef decltype(C2().x) T;
-    static_assert(96 % L == 0, "twiddles of a divisor of 96 points");
-    m = (m * (96 / L)) % 96;
-    const int quad = m / 24, r = m % 24;  // angle = quad * 90 degrees + r
-    T c, s;
-    if (r > 12) octant96<T>(24 - r, s, c);
-    else octant96<T>(r, c, s);
-    const T cv = quad == 0 ? c : (quad == 1 ? -s : (quad == 2 ? -c : s));
-    const T sv = quad == 0 ? s : (quad == 1 ? c : (quad == 2 ? -s : -c));
-    return cmul(a, mk<C2>(cv, sign < 0 ? -sv : sv));
-}
-
 // DFT of compile-time length L in registers; tw: the table of NL points
 // (w_L^m = tw[m * (NL/L)]) for radices 5 and 32.
 template <typename C2, int L, int NL>

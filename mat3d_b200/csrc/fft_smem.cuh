@@ -12,8 +12,10 @@
 //     b[(j/Ns)*Ns*R + (j mod Ns) + r*Ns] = v[r]
 // Twiddles come from a per-length table tw[m] = exp(-2 pi i m / n) in shared
 // memory (computed on the host in long double); the inverse uses conj().
-// Radices 2, 3, 4, 5 and 8 have dedicated butterflies; any other factor
-// (e.g. 13 for n = 65) uses a direct O(R^2) DFT through the table.
+// Radices 2 ... 16 of the factors 2, 3 and 5 have dedicated register DFTs, odd
+// primes up to 31 (e.g. 13 for n = 65) paired-input butterflies.  Plans take as
+// few stages as these radices allow (75 = 15 x 5): every stage costs a shared
+// read and write of each point and a barrier.
 //
 // Line addressing is two-level so one routine serves every pass layout:
 //     element e of line L lives at  (L / lpg) * gstride + (L % lpg) * lstride + e * estride
@@ -28,11 +30,55 @@ namespace m3d {
 
 constexpr int kMaxStages = 12;
 
+// x / d for 0 <= x, 1 <= d with x * d < 2^32 (always true for indices of a
+// shared-memory tile): round-up reciprocal m = ceil(2^32 / d), q = hi32(x m).
+// The error of x m / 2^32 against x / d is below x / 2^32 < 1 / d, too small
+// to carry the quotient past the next integer.
+struct FastDiv {
+    unsigned m;
+    int d;
+    __host__ __device__ __forceinline__ void init(int dd) {
+        d = dd;
+        m = dd > 1 ? 0xFFFFFFFFu / (unsigned)dd + 1u : 0u;
+    }
+    __device__ __forceinline__ int div(int x) const { return d == 1 ? x : (int)__umulhi((unsigned)x, m); }
+};
+inline FastDiv fast_div(int d) {
+    FastDiv f;
+    f.init(d);
+    return f;
+}
+
+// per-stage constants shared by every butterfly of a Stockham stage, made on
+// the host: a thread runs a handful of butterflies per stage, too few to pay
+// for two integer divisions each time
+struct StageIdx {
+    int R;       // radix
+    int step;    // n / (Ns R): twiddle index step
+    FastDiv nb;  // n / R: butterflies per line, and the input stride
+    FastDiv Ns;  // product of the earlier radices
+};
+
 struct LinePlan {
     int n;
     int nstages;
     int radix[kMaxStages];
+    StageIdx st[kMaxStages];
+    FastDiv dn;  // by n
 };
+// the derived constants of a plan whose n and radices are set
+inline void finish_plan(LinePlan& p) {
+    p.dn.init(p.n);
+    int Ns = 1;
+    for (int s = 0; s < p.nstages; ++s) {
+        const int R = p.radix[s];
+        p.st[s].R = R;
+        p.st[s].nb.init(p.n / R);
+        p.st[s].Ns.init(Ns);
+        p.st[s].step = p.n / R / Ns;
+        Ns *= R;
+    }
+}
 
 template <typename T> struct Cx;
 template <> struct Cx<float> { typedef float2 t; };
@@ -56,26 +102,46 @@ template <typename C2> __device__ __forceinline__ C2 twid(const C2* tw, int m, i
     return w;
 }
 
-// x / d for 0 <= x, 1 <= d with x * d < 2^32 (always true for indices of a
-// shared-memory tile): round-up reciprocal m = ceil(2^32 / d), q = hi32(x m).
-// The error of x m / 2^32 against x / d is below x / 2^32 < 1 / d, too small
-// to carry the quotient past the next integer.
-struct FastDiv {
-    unsigned m;
-    int d;
-    __device__ __forceinline__ void init(int dd) {
-        d = dd;
-        m = dd > 1 ? 0xFFFFFFFFu / (unsigned)dd + 1u : 0u;
+// exp(-+2 pi i m / L) for L dividing 96, m known at compile time: the sub-DFT
+// twiddles inside the register DFTs.  As immediates they cost neither the
+// broadcast shared-memory loads nor the registers of table entries (a radix-24
+// DFT multiplies by 15 of them); thermal 128^3 refinement 11.44 -> 11.33 ms a
+// solve.  Not for the radix-32 DFT, whose y forward pass at FP32 256^3 went from
+// 102 to 155 us with them.  cos and sin of
+// 2 pi k / 96 in the first octant, mirrored into the others; the switches fold
+// away once the loops over m are unrolled.
+template <typename T>
+__device__ __forceinline__ void octant96(int k, T& c, T& s) {
+    switch (k) {
+        case 0: c = (T)1.0000000000000000000000; s = (T)0.0; break;
+        case 1: c = (T)0.9978589232386035067380; s = (T)0.0654031292301430668153; break;
+        case 2: c = (T)0.9914448613738104111445; s = (T)0.1305261922200515915484; break;
+        case 3: c = (T)0.9807852804032304491261; s = (T)0.1950903220161282678482; break;
+        case 4: c = (T)0.9659258262890682867497; s = (T)0.2588190451025207623488; break;
+        case 5: c = (T)0.9469301294951056642558; s = (T)0.3214394653031615807010; break;
+        case 6: c = (T)0.9238795325112867561281; s = (T)0.3826834323650897717284; break;
+        case 7: c = (T)0.8968727415326883038941; s = (T)0.4422886902190012819952; break;
+        case 8: c = (T)0.8660254037844386467637; s = (T)0.5000000000000000000000; break;
+        case 9: c = (T)0.8314696123025452370787; s = (T)0.5555702330196022247428; break;
+        case 10: c = (T)0.7933533402912351645797; s = (T)0.6087614290087206394160; break;
+        case 11: c = (T)0.7518398074789773964075; s = (T)0.6593458151000688684251; break;
+        default: c = (T)0.7071067811865475244008; s = (T)0.7071067811865475244008; break;
     }
-    __device__ __forceinline__ int div(int x) const { return d == 1 ? x : (int)__umulhi((unsigned)x, m); }
-};
-
-// per-stage constants shared by every butterfly of a Stockham stage
-struct StageIdx {
-    int nb;    // n / R: butterflies per line, and the input stride
-    int Ns;    // product of the earlier radices
-    int step;  // n / (Ns R): twiddle index step
-};
+}
+// a * exp(sign 2 pi i m / L)
+template <typename C2, int L>
+__device__ __forceinline__ C2 rot_const(C2 a, int m, int sign) {
+    typedef decltype(C2().x) T;
+    static_assert(96 % L == 0, "twiddles of a divisor of 96 points");
+    m = (m * (96 / L)) % 96;
+    const int quad = m / 24, r = m % 24;  // angle = quad * 90 degrees + r
+    T c, s;
+    if (r > 12) octant96<T>(24 - r, s, c);
+    else octant96<T>(r, c, s);
+    const T cv = quad == 0 ? c : (quad == 1 ? -s : (quad == 2 ? -c : s));
+    const T sv = quad == 0 ? s : (quad == 1 ? c : (quad == 2 ? -s : -c));
+    return cmul(a, mk<C2>(cv, sign < 0 ? -sv : sv));
+}
 
 template <typename C2, int R>
 __device__ __forceinline__ void dft_small(C2 (&v)[R], const C2* tw, int n, int sign) {
@@ -136,6 +202,75 @@ __device__ __forceinline__ void dft_small(C2 (&v)[R], const C2* tw, int n, int s
         v[0] = cadd(a, t1);
         v[1] = cadd(t2, t3r);
         v[2] = csub(t2, t3r);
+    } else if constexpr (R == 5) {
+        // cos and sin of 72 and 144 degrees
+        const T c1 = (T)0.309016994374947424102293417182819L, c2 = (T)-0.809016994374947424102293417182819L;
+        const T sg = (T)(sign < 0 ? -1 : 1);
+        const T s1 = (T)0.951056516295153572116439333379382L * sg, s2 = (T)0.587785252292473129168705954639073L * sg;
+        const C2 a1 = cadd(v[1], v[4]), a2 = cadd(v[2], v[3]), b1 = csub(v[1], v[4]), b2 = csub(v[2], v[3]);
+        const C2 t1 = mk<C2>(v[0].x + c1 * a1.x + c2 * a2.x, v[0].y + c1 * a1.y + c2 * a2.y);
+        const C2 t2 = mk<C2>(v[0].x + c2 * a1.x + c1 * a2.x, v[0].y + c2 * a1.y + c1 * a2.y);
+        const C2 u1 = mk<C2>(s1 * b1.x + s2 * b2.x, s1 * b1.y + s2 * b2.y);
+        const C2 u2 = mk<C2>(s2 * b1.x - s1 * b2.x, s2 * b1.y - s1 * b2.y);
+        v[0] = cadd(v[0], cadd(a1, a2));
+        v[1] = mk<C2>(t1.x - u1.y, t1.y + u1.x);
+        v[4] = mk<C2>(t1.x + u1.y, t1.y - u1.x);
+        v[2] = mk<C2>(t2.x - u2.y, t2.y + u2.x);
+        v[3] = mk<C2>(t2.x + u2.y, t2.y - u2.x);
+    } else if constexpr (R == 9 || R == 16) {
+        // R = P x P: w_R twiddles between two rounds of P-point DFTs
+        constexpr int P = R == 9 ? 3 : 4;
+        C2 sub[P][P];
+#pragma unroll
+        for (int p = 0; p < P; ++p) {
+#pragma unroll
+            for (int m = 0; m < P; ++m) sub[p][m] = v[P * m + p];
+            dft_small<C2, P>(sub[p], tw, n, sign);
+        }
+#pragma unroll
+        for (int k1 = 0; k1 < P; ++k1) {
+            C2 t[P];
+#pragma unroll
+            for (int p = 0; p < P; ++p) {
+                if (p == 0 || k1 == 0) {
+                    t[p] = sub[p][k1];
+                } else if constexpr (R == 16) {
+                    t[p] = rot_const<C2, 16>(sub[p][k1], p * k1, sign);
+                } else {  // cos and sin of 40, 80 and 160 degrees
+                    const T c = p * k1 == 1 ? (T)0.766044443118978035202392650555417L
+                                            : (p * k1 == 2 ? (T)0.173648177666930348851716626769315L
+                                                           : (T)-0.939692620785908384054109277324731L);
+                    const T sn = p * k1 == 1 ? (T)0.642787609686539326322643409907263L
+                                             : (p * k1 == 2 ? (T)0.984807753012208059366743024589523L
+                                                            : (T)0.342020143325668733044099614682260L);
+                    t[p] = cmul(sub[p][k1], mk<C2>(c, sign < 0 ? -sn : sn));
+                }
+            }
+            dft_small<C2, P>(t, tw, n, sign);
+#pragma unroll
+            for (int k2 = 0; k2 < P; ++k2) v[k1 + P * k2] = t[k2];
+        }
+    } else if constexpr (R == 6 || R == 10 || R == 12 || R == 15) {
+        // R = P x Q, coprime: no twiddles between (Good's index maps)
+        constexpr int P = R == 12 ? 4 : (R == 15 ? 3 : 2), Q = R / P;
+        C2 sub[P][Q];
+#pragma unroll
+        for (int p = 0; p < P; ++p) {
+#pragma unroll
+            for (int q = 0; q < Q; ++q) sub[p][q] = v[(Q * p + P * q) % R];
+            dft_small<C2, Q>(sub[p], tw, n, sign);
+        }
+        // output k with k mod P = p, k mod Q = q: k = (p ep + q eq) mod R
+        constexpr int ep = R == 6 ? 3 : (R == 10 ? 5 : (R == 12 ? 9 : 10)), eq = R == 6 ? 4 : (R == 10 ? 6 : (R == 12 ? 4 : 6));
+#pragma unroll
+        for (int q = 0; q < Q; ++q) {
+            C2 t[P];
+#pragma unroll
+            for (int p = 0; p < P; ++p) t[p] = sub[p][q];
+            dft_small<C2, P>(t, tw, n, sign);
+#pragma unroll
+            for (int p = 0; p < P; ++p) v[(p * ep + q * eq) % R] = t[p];
+        }
     } else {
         // direct DFT through the table: w_R^m = tw[m * (n/R)]
         C2 in[R];
@@ -159,15 +294,15 @@ __device__ __forceinline__ void butterfly(const C2* __restrict__ src, C2* __rest
                                           const StageIdx& S, int es, const C2* tw, int sign) {
     C2 v[R];
 #pragma unroll
-    for (int r = 0; r < R; ++r) v[r] = src[(j + r * S.nb) * es];
-    if (S.Ns > 1) {
+    for (int r = 0; r < R; ++r) v[r] = src[(j + r * S.nb.d) * es];
+    if (S.Ns.d > 1) {
 #pragma unroll
         for (int r = 1; r < R; ++r) v[r] = cmul(v[r], twid(tw, k * r * S.step, sign));
     }
-    dft_small<C2, R>(v, tw, S.nb * R, sign);
-    const int idx = g * S.Ns * R + k;
+    dft_small<C2, R>(v, tw, S.nb.d * R, sign);
+    const int idx = g * S.Ns.d * R + k;
 #pragma unroll
-    for (int r = 0; r < R; ++r) dst[(idx + r * S.Ns) * es] = v[r];
+    for (int r = 0; r < R; ++r) dst[(idx + r * S.Ns.d) * es] = v[r];
 }
 
 // Odd radix R >= 5, compile time: inputs j and R-j are paired
@@ -183,7 +318,7 @@ __device__ __forceinline__ void butterfly_odd(const C2* __restrict__ src, C2* __
                                               const StageIdx& S, int es, const C2* tw, int sign) {
     typedef decltype(C2().x) T;
     constexpr int h = (R - 1) / 2;
-    const int nb = S.nb, Ns = S.Ns, step = S.step;
+    const int nb = S.nb.d, Ns = S.Ns.d, step = S.step;
     const C2 x0 = src[j * es];
     C2 a[h], b[h];
 #pragma unroll
@@ -230,9 +365,9 @@ __device__ __forceinline__ void butterfly_odd(const C2* __restrict__ src, C2* __
 constexpr int kMaxGenericRadix = 32;
 template <typename C2>
 __device__ __noinline__ void butterfly_generic(const C2* __restrict__ src, C2* __restrict__ dst, int R, int j, int g,
-                                               int k, StageIdx S, int es, const C2* tw, int sign) {
+                                               int k, const StageIdx& S, int es, const C2* tw, int sign) {
     typedef decltype(C2().x) T;
-    const int nb = S.nb, Ns = S.Ns, step = S.step;
+    const int nb = S.nb.d, Ns = S.Ns.d, step = S.step;
     C2 v[kMaxGenericRadix];
     for (int r = 0; r < R; ++r) v[r] = src[(j + r * nb) * es];
     for (int r = 1; r < R; ++r) v[r] = cmul(v[r], twid(tw, k * r * step, sign));
@@ -257,28 +392,25 @@ struct LineLayout {
 
 // Transforms every line; returns the buffer (a or b) that holds the result.
 // Must be called by all threads of the CTA; ends with __syncthreads().
-// Radices 2, 3, 4, 5, 8 are compile-time butterflies; odd radices 7..MaxR
-// (the primes and 9) are compile-time too when MaxR reaches them (each adds registers to the
-// kernel, so callers pick the smallest MaxR their lengths need); any other
-// radix runs the run-time generic butterfly.
+// Radices 2 ... 16 of the factors 2, 3 and 5 are compile-time butterflies; the
+// odd primes 7..MaxR are compile-time too when MaxR reaches them (each adds
+// registers to the kernel, so callers pick the smallest MaxR their lengths
+// need); any other radix runs the run-time generic butterfly.
 // one Stockham stage of radix R over every line of the tile (R fixed at
 // compile time, so the loop body is one straight-line butterfly); KIND 0 =
 // butterfly (2, 3, 4, 8), 1 = butterfly_odd, 2 = run-time generic
 template <typename C2, int R, int KIND>
 __device__ __forceinline__ void run_stage(const C2* a, C2* b, const C2* tw, const StageIdx& S, int Rrt,
                                           const LineLayout& L, const FastDiv& dl, const FastDiv& dg, int sign) {
-    FastDiv dnb, dns;
-    dnb.init(S.nb);
-    dns.init(S.Ns);
-    const int total = S.nb * L.nlines;
+    const int total = S.nb.d * L.nlines;
     const int es = L.estride;
     for (int w = threadIdx.x; w < total; w += blockDim.x) {
         int line, j;
         if (L.lines_fast) { j = dl.div(w); line = w - j * L.nlines; }
-        else { line = dnb.div(w); j = w - line * S.nb; }
+        else { line = S.nb.div(w); j = w - line * S.nb.d; }
         const int grp = dg.div(line);
         const int base = grp * L.gstride + (line - grp * L.lpg) * L.lstride;
-        const int g = dns.div(j), k = j - g * S.Ns;
+        const int g = S.Ns.div(j), k = j - g * S.Ns.d;
         if constexpr (KIND == 0) butterfly<C2, R>(a + base, b + base, j, g, k, S, es, tw, sign);
         else if constexpr (KIND == 1) butterfly_odd<C2, R>(a + base, b + base, j, g, k, S, es, tw, sign);
         else butterfly_generic<C2>(a + base, b + base, Rrt, j, g, k, S, es, tw, sign);
@@ -286,27 +418,28 @@ __device__ __forceinline__ void run_stage(const C2* a, C2* b, const C2* tw, cons
 }
 
 template <typename C2, int MaxR = 5>
-__device__ C2* fft_lines(C2* a, C2* b, const C2* tw, const LinePlan& p, const LineLayout& L, int sign) {
+__device__ __forceinline__ C2* fft_lines(C2* a, C2* b, const C2* tw, const LinePlan& p, const LineLayout& L, int sign) {
     const int n = p.n;
     FastDiv dl, dg;  // by the lines of the tile, by the lines of a group
     dl.init(L.nlines);
     dg.init(L.lpg);
-    int Ns = 1;
     for (int s = 0; s < p.nstages; ++s) {
-        const int R = p.radix[s];
-        StageIdx S;
-        S.nb = n / R;
-        S.Ns = Ns;
-        S.step = S.nb / Ns;
+        const StageIdx& S = p.st[s];
+        const int R = S.R;
         switch (R) {
             case 2: run_stage<C2, 2, 0>(a, b, tw, S, R, L, dl, dg, sign); break;
             case 3: run_stage<C2, 3, 0>(a, b, tw, S, R, L, dl, dg, sign); break;
             case 4: run_stage<C2, 4, 0>(a, b, tw, S, R, L, dl, dg, sign); break;
-            case 5: run_stage<C2, 5, 1>(a, b, tw, S, R, L, dl, dg, sign); break;
+            case 5: run_stage<C2, 5, 0>(a, b, tw, S, R, L, dl, dg, sign); break;
+            case 6: run_stage<C2, 6, 0>(a, b, tw, S, R, L, dl, dg, sign); break;
             case 8: run_stage<C2, 8, 0>(a, b, tw, S, R, L, dl, dg, sign); break;
+            case 9: run_stage<C2, 9, 0>(a, b, tw, S, R, L, dl, dg, sign); break;
+            case 10: run_stage<C2, 10, 0>(a, b, tw, S, R, L, dl, dg, sign); break;
+            case 12: run_stage<C2, 12, 0>(a, b, tw, S, R, L, dl, dg, sign); break;
+            case 15: run_stage<C2, 15, 0>(a, b, tw, S, R, L, dl, dg, sign); break;
+            case 16: run_stage<C2, 16, 0>(a, b, tw, S, R, L, dl, dg, sign); break;
             default:
                 if constexpr (MaxR >= 7) if (R == 7) { run_stage<C2, 7, 1>(a, b, tw, S, R, L, dl, dg, sign); break; }
-                if constexpr (MaxR >= 9) if (R == 9) { run_stage<C2, 9, 1>(a, b, tw, S, R, L, dl, dg, sign); break; }
                 if constexpr (MaxR >= 11) if (R == 11) { run_stage<C2, 11, 1>(a, b, tw, S, R, L, dl, dg, sign); break; }
                 if constexpr (MaxR >= 13) if (R == 13) { run_stage<C2, 13, 1>(a, b, tw, S, R, L, dl, dg, sign); break; }
                 if constexpr (MaxR >= 17) if (R == 17) { run_stage<C2, 17, 1>(a, b, tw, S, R, L, dl, dg, sign); break; }
@@ -319,7 +452,6 @@ __device__ C2* fft_lines(C2* a, C2* b, const C2* tw, const LinePlan& p, const Li
         }
         __syncthreads();
         C2* t = a; a = b; b = t;
-        Ns *= R;
     }
     return a;
 }

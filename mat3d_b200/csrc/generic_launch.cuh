@@ -47,7 +47,7 @@ void allow_smem(K kernel) {
 inline int max_radix(const LinePlan& p) {
     int r = 5;
     for (int s = 0; s < p.nstages; ++s)
-        if (p.radix[s] % 2 == 1 && p.radix[s] > r) r = p.radix[s];
+        if (p.radix[s] % 2 && p.radix[s] % 3 && p.radix[s] % 5 && p.radix[s] > r) r = p.radix[s];  // a prime above 5
     return r <= 5 ? 5 : (r <= 13 ? 13 : 31);
 }
 template <int R> struct RadixC { static constexpr int value = R; };
@@ -60,44 +60,44 @@ template <class F> void with_radix(const LinePlan& p, F&& f) {
 }
 
 template <int MaxR, typename T, int C, class Pro>
-void gen_zfwd(dim3 grid, size_t smem, cudaStream_t st, const GridDims& g, const LinePlan& p,
+void gen_zfwd(dim3 grid, int nt, size_t smem, cudaStream_t st, const GridDims& g, const LinePlan& p,
               const typename Cx<T>::t* tw, typename Cx<T>::t* sp, const Pro& pro, const Ctl* ctl, int G, double* part) {
     allow_smem(k_zfwd<T, C, Pro, MaxR>);
-    k_zfwd<T, C, Pro, MaxR><<<grid, 256, smem, st>>>(g, p, tw, sp, pro, ctl, G, part);
+    k_zfwd<T, C, Pro, MaxR><<<grid, nt, smem, st>>>(g, p, tw, sp, pro, ctl, G, part);
 }
 template <int MaxR, typename T>
-void gen_y(dim3 grid, size_t smem, cudaStream_t st, const GridDims& g, const LinePlan& p,
-           const typename Cx<T>::t* tw, typename Cx<T>::t* sp, int tz, int CC, int sign, const Ctl* ctl) {
+void gen_y(dim3 grid, int nt, size_t smem, cudaStream_t st, const GridDims& g, const LinePlan& p,
+           const typename Cx<T>::t* tw, typename Cx<T>::t* sp, FastDiv tz, FastDiv ntz, int CC, int sign, const Ctl* ctl) {
     allow_smem(k_ypass<T, MaxR>);
-    k_ypass<T, MaxR><<<grid, 256, smem, st>>>(g, p, tw, sp, tz, CC, sign, ctl);
+    k_ypass<T, MaxR><<<grid, nt, smem, st>>>(g, p, tw, sp, tz, ntz, CC, sign, ctl);
 }
 template <int MaxR, typename T, int C, class Spec>
-void gen_x(dim3 grid, size_t smem, cudaStream_t st, const GridDims& g, const LinePlan& p,
-           const typename Cx<T>::t* tw, typename Cx<T>::t* sp, int tz, const Spec& op, const Ctl* ctl, double* part) {
+void gen_x(dim3 grid, int nt, size_t smem, cudaStream_t st, const GridDims& g, const LinePlan& p,
+           const typename Cx<T>::t* tw, typename Cx<T>::t* sp, FastDiv tz, FastDiv ntz, const Spec& op, const Ctl* ctl, double* part) {
     allow_smem(k_xturn<T, C, Spec, MaxR>);
-    k_xturn<T, C, Spec, MaxR><<<grid, 256, smem, st>>>(g, p, tw, sp, tz, op, ctl, part);
+    k_xturn<T, C, Spec, MaxR><<<grid, nt, smem, st>>>(g, p, tw, sp, tz, ntz, op, ctl, part);
 }
 template <int MaxR, typename T, int C, class Epi, class Fin>
-void gen_zinv(dim3 grid, size_t smem, cudaStream_t st, const GridDims& g, const LinePlan& p,
+void gen_zinv(dim3 grid, int nt, size_t smem, cudaStream_t st, const GridDims& g, const LinePlan& p,
               const typename Cx<T>::t* tw, const typename Cx<T>::t* sp, const Epi& epi, Ctl* ctl, int G, double* part,
               const Fin& fin) {
     allow_smem(k_zinv<T, C, Epi, Fin, MaxR>);
-    k_zinv<T, C, Epi, Fin, MaxR><<<grid, 256, smem, st>>>(g, p, tw, sp, epi, ctl, G, part, fin);
+    k_zinv<T, C, Epi, Fin, MaxR><<<grid, nt, smem, st>>>(g, p, tw, sp, epi, ctl, G, part, fin);
 }
 
 // every generic launch the solver makes, for one MaxR (explicit instantiation
 // declarations and definitions)
 #define M3D_GEN_ZFWD(EXT, R, T, C, PRO)                                                                              \
-    EXT template void gen_zfwd<R, T, C, PRO>(dim3, size_t, cudaStream_t, const GridDims&, const LinePlan&,           \
+    EXT template void gen_zfwd<R, T, C, PRO>(dim3, int, size_t, cudaStream_t, const GridDims&, const LinePlan&,           \
                                              const Cx<T>::t*, Cx<T>::t*, const PRO&, const Ctl*, int, double*);
 #define M3D_GEN_Y(EXT, R, T)                                                                                         \
-    EXT template void gen_y<R, T>(dim3, size_t, cudaStream_t, const GridDims&, const LinePlan&, const Cx<T>::t*,     \
-                                  Cx<T>::t*, int, int, int, const Ctl*);
+    EXT template void gen_y<R, T>(dim3, int, size_t, cudaStream_t, const GridDims&, const LinePlan&, const Cx<T>::t*,     \
+                                  Cx<T>::t*, FastDiv, FastDiv, int, int, const Ctl*);
 #define M3D_GEN_X(EXT, R, T, C, SPEC)                                                                                \
-    EXT template void gen_x<R, T, C, SPEC>(dim3, size_t, cudaStream_t, const GridDims&, const LinePlan&,             \
-                                           const Cx<T>::t*, Cx<T>::t*, int, const SPEC&, const Ctl*, double*);
+    EXT template void gen_x<R, T, C, SPEC>(dim3, int, size_t, cudaStream_t, const GridDims&, const LinePlan&,             \
+                                           const Cx<T>::t*, Cx<T>::t*, FastDiv, FastDiv, const SPEC&, const Ctl*, double*);
 #define M3D_GEN_ZINV(EXT, R, T, C, EPI, FIN)                                                                         \
-    EXT template void gen_zinv<R, T, C, EPI, FIN>(dim3, size_t, cudaStream_t, const GridDims&, const LinePlan&,      \
+    EXT template void gen_zinv<R, T, C, EPI, FIN>(dim3, int, size_t, cudaStream_t, const GridDims&, const LinePlan&,      \
                                                   const Cx<T>::t*, const Cx<T>::t*, const EPI&, Ctl*, int, double*,  \
                                                   const FIN&);
 typedef ProMat<float, 3> GPm3f; typedef ProMat<float, 6> GPm6f; typedef ProMat<double, 3> GPm3d; typedef ProMat<double, 6> GPm6d;

@@ -71,6 +71,7 @@ bool plan_of(int n, LinePlan& p) {
     p.n = n;
     p.nstages = (int)f.size();
     for (int i = 0; i < kMaxStages; ++i) p.radix[i] = i < (int)f.size() ? f[i] : 1;
+    finish_plan(p);
     return true;
 }
 
@@ -133,6 +134,8 @@ extern "C" int m3d_thermal_solve_noalloc(int Nx, int Ny, int Nz, double km, doub
     g.Nx = Nx; g.Ny = Ny; g.Nz = Nz;
     g.Hz = Nz / 2 + 1;
     g.Hzp = (g.Hz + 1) & ~1;
+    g.dHz.init(g.Hz);
+    g.dHzp.init(g.Hzp);
     g.V = (long long)Nx * Ny * Nz;
     g.NL = (long long)Nx * Ny;
     constexpr int C = 3;
@@ -262,6 +265,7 @@ extern "C" int m3d_thermal_solve_noalloc(int Nx, int Ny, int Nz, double km, doub
     const size_t ysmem = (size_t)Ny * sizeof(double2) + 2 * (size_t)Ny * TZy * sizeof(double2);
     const size_t xsmem = (size_t)Nx * sizeof(double2) + 2 * (size_t)C * Nx * TZx * sizeof(double2) + 16 + 32 * 32 * 8;
     const int ntzy = (g.Hzp + TZy - 1) / TZy, ntzx = (g.Hzp + TZx - 1) / TZx;
+    const FastDiv dTZy = fast_div(TZy), dTZx = fast_div(TZx), dntzy = fast_div(ntzy), dntzx = fast_div(ntzx);
     {
         std::lock_guard<std::mutex> lk(g_noalloc_mu);  // kernel attributes are per device
         if (!g_noalloc_attrs[dev]) {
@@ -278,9 +282,9 @@ extern "C" int m3d_thermal_solve_noalloc(int Nx, int Ny, int Nz, double km, doub
     for (;;) {
         for (int k = 0; k < 8; ++k) {
             k_zfwd<double, C, ProMat<double, C>, 5><<<dim3(zblk, 1), 256, zsmem, stream>>>(g, pz, twz, spec, pro, ctl, G, part);
-            k_ypass<double, 5><<<dim3(Nx * ntzy, C), 256, ysmem, stream>>>(g, py, twy, spec, TZy, C, -1, ctl);
-            k_xturn<double, C, SpecGreen<double, C>, 5><<<dim3(Ny * ntzx, 1), 256, xsmem, stream>>>(g, px, twx, spec, TZx, sg, ctl, part);
-            k_ypass<double, 5><<<dim3(Nx * ntzy, C), 256, ysmem, stream>>>(g, py, twy, spec, TZy, C, +1, ctl);
+            k_ypass<double, 5><<<dim3(Nx * ntzy, C), 256, ysmem, stream>>>(g, py, twy, spec, dTZy, dntzy, C, -1, ctl);
+            k_xturn<double, C, SpecGreen<double, C>, 5><<<dim3(Ny * ntzx, 1), 256, xsmem, stream>>>(g, px, twx, spec, dTZx, dntzx, sg, ctl, part);
+            k_ypass<double, 5><<<dim3(Nx * ntzy, C), 256, ysmem, stream>>>(g, py, twy, spec, dTZy, dntzy, C, +1, ctl);
             k_zinv<double, C, EpiEM<double, C>, FinLinear, 5><<<dim3(zblk, 1), 256, zsmem, stream>>>(g, pz, twz, spec, epi, ctl, G, part, fin);
         }
         NA_CUDA(cudaGetLastError());

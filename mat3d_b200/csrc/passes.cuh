@@ -21,6 +21,7 @@ namespace m3d {
 
 struct GridDims {
     int Nx, Ny, Nz, Hz, Hzp;
+    FastDiv dHz, dHzp;  // by Hz and Hzp (the generic passes' index splits)
     long long V;   // Nx*Ny*Nz
     long long NL;  // Nx*Ny (z lines)
     // compacted launches: live[0] = number of entries still iterating,
@@ -129,7 +130,7 @@ __device__ __forceinline__ char* align_up(char* p, int a) {
 // as one complex line -> FFT along z -> split into two half spectra.
 // ============================================================================
 template <typename T, int C, class Pro, int MaxR>
-__global__ void __launch_bounds__(256) k_zfwd(GridDims g, LinePlan pz, const typename Cx<T>::t* __restrict__ twz,
+__global__ void __launch_bounds__(256) k_zfwd(GridDims g, const __grid_constant__ LinePlan pz, const typename Cx<T>::t* __restrict__ twz,
                                               typename Cx<T>::t* __restrict__ spec, Pro pro, const Ctl* __restrict__ ctl,
                                               int G, double* partials) {
     typedef typename Cx<T>::t C2;
@@ -153,7 +154,7 @@ __global__ void __launch_bounds__(256) k_zfwd(GridDims g, LinePlan pz, const typ
     const long long l0 = (long long)blockIdx.x * G;
     double acc[Pro::NSUM > 0 ? Pro::NSUM : 1] = {};
     for (int i = threadIdx.x; i < G * Nz; i += blockDim.x) {
-        const int gi = i / Nz, z = i - gi * Nz;
+        const int gi = pz.dn.div(i), z = i - gi * Nz;
         const long long l = l0 + gi;
         T val[C];
         if (l < g.NL) {
@@ -173,7 +174,7 @@ __global__ void __launch_bounds__(256) k_zfwd(GridDims g, LinePlan pz, const typ
 
     const int Hz = g.Hz, Hzp = g.Hzp;
     for (int i = threadIdx.x; i < nl * Hzp; i += blockDim.x) {
-        const int k = i % Hzp, pc = i / Hzp;
+        const int pc = g.dHzp.div(i), k = i - pc * Hzp;
         const int p = pc / C, c = pc - p * C;
         const long long la = l0 + 2 * p, lb = la + 1;
         C2 Av = mk<C2>(0, 0), Bv = mk<C2>(0, 0);
@@ -197,32 +198,31 @@ __global__ void __launch_bounds__(256) k_zfwd(GridDims g, LinePlan pz, const typ
 // CTA = one x, TZ consecutive kz columns, one (batch, component).
 // ============================================================================
 template <typename T, int MaxR>
-__global__ void __launch_bounds__(256) k_ypass(GridDims g, LinePlan py, const typename Cx<T>::t* __restrict__ twy,
-                                               typename Cx<T>::t* __restrict__ spec, int TZ, int C, int sign,
-                                               const Ctl* __restrict__ ctl) {
+__global__ void __launch_bounds__(256) k_ypass(GridDims g, const __grid_constant__ LinePlan py, const typename Cx<T>::t* __restrict__ twy,
+                                               typename Cx<T>::t* __restrict__ spec, FastDiv dTZ, FastDiv dntz,
+                                               int C, int sign, const Ctl* __restrict__ ctl) {
     typedef typename Cx<T>::t C2;
     const int b = entry_of(g, blockIdx.y / C);
     if (b < 0 || ctl[b].done) return;
     const int cb = b * C + blockIdx.y % C;
     extern __shared__ __align__(16) char smem_raw[];
-    const int Ny = g.Ny, Hzp = g.Hzp;
+    const int Ny = g.Ny, Hzp = g.Hzp, TZ = dTZ.d;
     C2* tw = (C2*)smem_raw;
     C2* A = tw + Ny;
     C2* B = A + (size_t)Ny * TZ;
     for (int i = threadIdx.x; i < Ny; i += blockDim.x) tw[i] = twy[i];
-    const int ntz = (Hzp + TZ - 1) / TZ;
-    const int x = blockIdx.x / ntz, kz0 = (blockIdx.x - x * ntz) * TZ;
+    const int x = dntz.div(blockIdx.x), kz0 = (blockIdx.x - x * dntz.d) * TZ;
     C2* base = spec + ((long long)cb * g.NL + (long long)x * Ny) * Hzp + kz0;
     for (int i = threadIdx.x; i < Ny * TZ; i += blockDim.x) {
-        const int y = i / TZ, col = i - y * TZ;
-        A[i] = (kz0 + col < Hzp) ? base[(long long)y * Hzp + col] : mk<C2>(0, 0);
+        const int y = dTZ.div(i), col = i - y * TZ;
+        A[i] = (kz0 + col < Hzp) ? base[y * Hzp + col] : mk<C2>(0, 0);
     }
     __syncthreads();
     LineLayout L{TZ, TZ, 1, 0, TZ, true};
     C2* R = fft_lines<C2, MaxR>(A, B, tw, py, L, sign);
     for (int i = threadIdx.x; i < Ny * TZ; i += blockDim.x) {
-        const int y = i / TZ, col = i - y * TZ;
-        if (kz0 + col < Hzp) base[(long long)y * Hzp + col] = R[i];
+        const int y = dTZ.div(i), col = i - y * TZ;
+        if (kz0 + col < Hzp) base[y * Hzp + col] = R[i];
     }
 }
 
@@ -232,28 +232,26 @@ __global__ void __launch_bounds__(256) k_ypass(GridDims g, LinePlan py, const ty
 //   optional reductions) -> inverse FFT along x (when Spec::kInverse).
 // ============================================================================
 template <typename T, int C, class Spec, int MaxR>
-__global__ void __launch_bounds__(256) k_xturn(GridDims g, LinePlan px, const typename Cx<T>::t* __restrict__ twx,
-                                               typename Cx<T>::t* __restrict__ spec, int TZ, Spec op,
-                                               const Ctl* __restrict__ ctl, double* partials) {
+__global__ void __launch_bounds__(256) k_xturn(GridDims g, const __grid_constant__ LinePlan px, const typename Cx<T>::t* __restrict__ twx,
+                                               typename Cx<T>::t* __restrict__ spec, FastDiv dTZ, FastDiv dntz,
+                                               Spec op, const Ctl* __restrict__ ctl, double* partials) {
     typedef typename Cx<T>::t C2;
     const int b = entry_of(g, blockIdx.y);
     if (b < 0 || ctl[b].done) return;
     op.prepare(ctl, b);
     extern __shared__ __align__(16) char smem_raw[];
-    const int Nx = g.Nx, Ny = g.Ny, Hzp = g.Hzp;
+    const int Nx = g.Nx, Ny = g.Ny, Hzp = g.Hzp, TZ = dTZ.d;
     C2* tw = (C2*)smem_raw;
     C2* A = tw + Nx;
     C2* B = A + (size_t)C * Nx * TZ;
     double* red = (double*)align_up((char*)(B + (size_t)C * Nx * TZ), 16);
     for (int i = threadIdx.x; i < Nx; i += blockDim.x) tw[i] = twx[i];
-    const int ntz = (Hzp + TZ - 1) / TZ;
-    const int y = blockIdx.x / ntz, kz0 = (blockIdx.x - y * ntz) * TZ;
+    const int y = dntz.div(blockIdx.x), kz0 = (blockIdx.x - y * dntz.d) * TZ;
+    C2* base = spec + ((long long)b * C * g.NL + y) * Hzp + kz0;
     for (int i = threadIdx.x; i < C * Nx * TZ; i += blockDim.x) {
-        const int col = i % TZ, r = i / TZ;
-        const int x = r % Nx, c = r / Nx;
-        A[i] = (kz0 + col < Hzp)
-                   ? spec[(((long long)b * C + c) * g.NL + (long long)x * Ny + y) * Hzp + kz0 + col]
-                   : mk<C2>(0, 0);
+        const int r = dTZ.div(i), col = i - r * TZ;
+        const int c = px.dn.div(r), x = r - c * Nx;
+        A[i] = (kz0 + col < Hzp) ? base[((long long)c * g.NL + (long long)x * Ny) * Hzp + col] : mk<C2>(0, 0);
     }
     __syncthreads();
     LineLayout L{C * TZ, TZ, 1, Nx * TZ, TZ, true};
@@ -262,7 +260,7 @@ __global__ void __launch_bounds__(256) k_xturn(GridDims g, LinePlan px, const ty
 
     double acc[Spec::NSUM > 0 ? Spec::NSUM : 1] = {};
     for (int i = threadIdx.x; i < Nx * TZ; i += blockDim.x) {
-        const int col = i % TZ, x = i / TZ;
+        const int x = dTZ.div(i), col = i - x * TZ;
         const int kz = kz0 + col;
         if (kz >= g.Hz) continue;
         C2 v[C];
@@ -281,10 +279,9 @@ __global__ void __launch_bounds__(256) k_xturn(GridDims g, LinePlan px, const ty
         __syncthreads();
         C2* Q = fft_lines<C2, MaxR>(R, S, tw, px, L, +1);
         for (int i = threadIdx.x; i < C * Nx * TZ; i += blockDim.x) {
-            const int col = i % TZ, r = i / TZ;
-            const int x = r % Nx, c = r / Nx;
-            if (kz0 + col < Hzp)
-                spec[(((long long)b * C + c) * g.NL + (long long)x * Ny + y) * Hzp + kz0 + col] = Q[i];
+            const int r = dTZ.div(i), col = i - r * TZ;
+            const int c = px.dn.div(r), x = r - c * Nx;
+            if (kz0 + col < Hzp) base[((long long)c * g.NL + (long long)x * Ny) * Hzp + col] = Q[i];
         }
     }
 }
@@ -295,7 +292,7 @@ __global__ void __launch_bounds__(256) k_xturn(GridDims g, LinePlan px, const ty
 // real parts / imaginary parts are the two real lines -> epilogue per voxel.
 // ============================================================================
 template <typename T, int C, class Epi, class Fin, int MaxR>
-__global__ void __launch_bounds__(256) k_zinv(GridDims g, LinePlan pz, const typename Cx<T>::t* __restrict__ twz,
+__global__ void __launch_bounds__(256) k_zinv(GridDims g, const __grid_constant__ LinePlan pz, const typename Cx<T>::t* __restrict__ twz,
                                               const typename Cx<T>::t* __restrict__ spec, Epi epi, Ctl* ctl, int G,
                                               double* partials, Fin fin) {
     typedef typename Cx<T>::t C2;
@@ -316,7 +313,7 @@ __global__ void __launch_bounds__(256) k_zinv(GridDims g, LinePlan pz, const typ
     epi.load_smem(extra, b);
     const long long l0 = (long long)blockIdx.x * G;
     for (int i = threadIdx.x; i < nl * Hz; i += blockDim.x) {
-        const int k = i % Hz, pc = i / Hz;
+        const int pc = g.dHz.div(i), k = i - pc * Hz;
         const int p = pc / C, c = pc - p * C;
         const long long la = l0 + 2 * p, lb = la + 1;
         const long long rowbase = ((long long)b * C + c) * g.NL;
@@ -338,7 +335,7 @@ __global__ void __launch_bounds__(256) k_zinv(GridDims g, LinePlan pz, const typ
     const T invV = (T)(1.0 / (double)g.V);
     double acc[Epi::NSUM > 0 ? Epi::NSUM : 1] = {};
     for (int i = threadIdx.x; i < G * Nz; i += blockDim.x) {
-        const int gi = i / Nz, z = i - gi * Nz;
+        const int gi = pz.dn.div(i), z = i - gi * Nz;
         const long long l = l0 + gi;
         if (l >= g.NL) continue;
         const int p = gi >> 1;

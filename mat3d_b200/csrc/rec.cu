@@ -148,7 +148,7 @@ enum ZMode { Z_FWD = 0, Z_RAND = 1, Z_INV = 2, Z_BWD = 3 };
 //   Z_BWD : A = unnormalised inverse FFT_z(m) (plain transforms)
 template <int MODE, int MaxR>
 __global__ void __launch_bounds__(kThreads) krec_z(double2* __restrict__ A, double2* __restrict__ m,
-                                                    const double2* __restrict__ twz, LinePlan pz, int G,
+                                                    const double2* __restrict__ twz, const __grid_constant__ LinePlan pz, int G,
                                                     long long nlines, int ntiles, const RecCtl* __restrict__ ctl) {
     if (MODE == Z_RAND && !restart_pass(ctl)) return;
     if (MODE == Z_INV && ctl->done) return;
@@ -273,7 +273,7 @@ enum YMode { Y_FWD = 0, Y_RAND = 1, Y_INV = 2 };
 // of a tile overlaps the arithmetic of the one before.
 template <int MODE, int MaxR>
 __global__ void __launch_bounds__(kThreads) krec_y(double2* __restrict__ A, const double2* __restrict__ twy,
-                                                    LinePlan py, int Nz, int TZ, int ntz, int ntiles,
+                                                    const __grid_constant__ LinePlan py, int Nz, int TZ, int ntz, int ntiles,
                                                     const RecCtl* __restrict__ ctl) {
     if (MODE == Y_RAND && !restart_pass(ctl)) return;
     if (MODE == Y_INV && ctl->done) return;
@@ -318,7 +318,7 @@ __global__ void __launch_bounds__(kThreads) krec_y(double2* __restrict__ A, cons
 enum XOut { XO_ANGLE = 0, XO_COPY = 1, XO_NORM = 2 };
 template <int OUT, int MaxR>
 __global__ void __launch_bounds__(kThreads) krec_xout(double2* __restrict__ A, double* __restrict__ R,
-                                                       const double2* __restrict__ twx, LinePlan px, int Ny, int Nz,
+                                                       const double2* __restrict__ twx, const __grid_constant__ LinePlan px, int Ny, int Nz,
                                                        int TZ, int ntz, int ntiles, int sign,
                                                        const RecCtl* __restrict__ ctl) {
     if (OUT == XO_ANGLE && !restart_pass(ctl)) return;
@@ -378,7 +378,7 @@ __global__ void __launch_bounds__(kThreads) krec_xout(double2* __restrict__ A, d
 template <int MaxR>
 __global__ void __launch_bounds__(kThreads) krec_xturn(double2* __restrict__ A, const double* __restrict__ normC,
                                                         const double* __restrict__ R, const double2* __restrict__ twx,
-                                                        LinePlan px, int Ny, int Nz, int TZ, int ntz, int ntiles,
+                                                        const __grid_constant__ LinePlan px, int Ny, int Nz, int TZ, int ntz, int ntiles,
                                                         double* __restrict__ part, double* __restrict__ errs,
                                                         RecCtl* ctl) {
     extern __shared__ __align__(16) char smem_raw[];
@@ -921,7 +921,7 @@ static int rec_alloc(int Nx, int Ny, int Nz, int device, m3d_rec** out) {
     h->Nx = Nx; h->Ny = Ny; h->Nz = Nz;
     h->xyz = (long long)Nx * Ny * Nz;
     h->device = device;
-    if (!make_plan(Nx, h->px, true) || !make_plan(Ny, h->py, true) || !make_plan(Nz, h->pz, true)) {
+    if (!make_plan(Nx, h->px) || !make_plan(Ny, h->py) || !make_plan(Nz, h->pz)) {
         delete h;
         return failr(M3D_ERR_UNSUPPORTED, "grid sizes need prime factors <= 32");
     }
@@ -974,7 +974,7 @@ static int rec_alloc(int Nx, int Ny, int Nz, int device, m3d_rec** out) {
     cudaMemset(h->d_ctl, 0, sizeof(RecCtl));
     int mr = 5;
     for (const LinePlan* pl : {&h->px, &h->py, &h->pz})
-        for (int k = 0; k < pl->nstages; ++k) mr = std::max(mr, pl->radix[k] == 8 ? 5 : pl->radix[k]);
+        for (int k = 0; k < pl->nstages; ++k) if (pl->radix[k] % 2 && pl->radix[k] % 3 && pl->radix[k] % 5) mr = std::max(mr, pl->radix[k]);  // a prime above 5
     h->maxr = mr <= 5 ? 5 : mr <= 13 ? 13 : mr <= 19 ? 19 : 31;
     h->set_smem();
     if (cudaDeviceSynchronize() != cudaSuccess || cudaGetLastError() != cudaSuccess) {

@@ -612,7 +612,7 @@ void m3d_solver::pass_zfwd(Pro pro, Ctl* ctl, typename Cx<T>::t* sp) {
         const int zblk = (int)((g.NL + Gl - 1) / Gl);
         const size_t zsmem = (size_t)Nz * sizeof(C2) + 2 * (size_t)(Gl / 2) * CC * Nz * sizeof(C2) + 16 + 32 * 32 * 8 + extra;
         with_radix(pz, [&](auto r) {
-            gen_zfwd<decltype(r)::value, T, CC, Pro>(dim3(zblk, gridB()), zsmem, stream, g, pz, tw<T>(2), sp, pro, ctl, Gl,
+            gen_zfwd<decltype(r)::value, T, CC, Pro>(dim3(zblk, gridB()), plan_threads(pz, Gl / 2 * CC), zsmem, stream, g, pz, tw<T>(2), sp, pro, ctl, Gl,
                                                      d_part);
         });
     }
@@ -712,7 +712,8 @@ void m3d_solver::pass_y(int sign, int CC, Ctl* ctl, typename Cx<T>::t* sp) {
         const size_t ysmem = (size_t)Ny * sizeof(C2) + 2 * (size_t)Ny * tzy * sizeof(C2);
         const int ntzy = (g.Hzp + tzy - 1) / tzy;
         with_radix(py, [&](auto r) {
-            gen_y<decltype(r)::value, T>(dim3(Nx * ntzy, CC * gridB()), ysmem, stream, g, py, tw<T>(1), sp, tzy, CC, sign, ctl);
+            gen_y<decltype(r)::value, T>(dim3(Nx * ntzy, CC * gridB()), plan_threads(py, tzy), ysmem, stream, g, py, tw<T>(1), sp,
+                                         fast_div(tzy), fast_div(ntzy), CC, sign, ctl);
         });
     }
     st.kernel_launches += 1;
@@ -790,7 +791,8 @@ int m3d_solver::pass_x(Spec op, Ctl* ctl, typename Cx<T>::t* sp) {
         const int ntzx = (g.Hzp + tzx - 1) / tzx;
         nblk = Ny * ntzx;
         with_radix(px, [&](auto r) {
-            gen_x<decltype(r)::value, T, CC, Spec>(dim3(nblk, gridB()), xsmem, stream, g, px, tw<T>(0), sp, tzx, op, ctl, d_part);
+            gen_x<decltype(r)::value, T, CC, Spec>(dim3(nblk, gridB()), plan_threads(px, CC * tzx), xsmem, stream, g, px, tw<T>(0), sp,
+                                                   fast_div(tzx), fast_div(ntzx), op, ctl, d_part);
         });
     }
     st.kernel_launches += 1;
@@ -815,7 +817,7 @@ int m3d_solver::pass_zinv(Epi epi, Ctl* ctl, typename Cx<T>::t* sp, Fin fin) {
         nblk = (int)((g.NL + Gl - 1) / Gl);
         const size_t zsmem = (size_t)Nz * sizeof(C2) + 2 * (size_t)(Gl / 2) * CC * Nz * sizeof(C2) + 16 + 32 * 32 * 8 + extra;
         with_radix(pz, [&](auto r) {
-            gen_zinv<decltype(r)::value, T, CC, Epi, Fin>(dim3(nblk, gridB()), zsmem, stream, g, pz, tw<T>(2), sp, epi, ctl, Gl,
+            gen_zinv<decltype(r)::value, T, CC, Epi, Fin>(dim3(nblk, gridB()), plan_threads(pz, Gl / 2 * CC), zsmem, stream, g, pz, tw<T>(2), sp, epi, ctl, Gl,
                                                           d_part, fin);
         });
     }
@@ -1642,12 +1644,14 @@ static int create_impl(int kind, int Nx, int Ny, int Nz, int behav, int precisio
     h->g.Nx = Nx; h->g.Ny = Ny; h->g.Nz = Nz;
     h->g.Hz = Nz / 2 + 1;
     h->g.Hzp = even_up(Nz / 2 + 1);
+    h->g.dHz.init(h->g.Hz);
+    h->g.dHzp.init(h->g.Hzp);
     h->g.V = (long long)Nx * Ny * Nz;
     h->g.NL = (long long)Nx * Ny;
     // M3D_FFT_SCHEDULE=<0..3>: the generic line FFTs' radix-stage order (make_plan)
     const char* esch = std::getenv("M3D_FFT_SCHEDULE");
     const int sched = esch ? std::max(0, std::min(kPlanOrders - 1, std::atoi(esch))) : 0;
-    if (!make_plan(Nx, h->px, false, sched) || !make_plan(Ny, h->py, false, sched) || !make_plan(Nz, h->pz, false, sched)) {
+    if (!make_plan(Nx, h->px, sched) || !make_plan(Ny, h->py, sched) || !make_plan(Nz, h->pz, sched)) {
         delete h;
         return fail(M3D_ERR_UNSUPPORTED, "grid sizes need prime factors <= 32");
     }
@@ -2344,10 +2348,10 @@ int m3d_solver::autotune(int sweeps, m3d_tune* out) {
         };
         for (int o = 1; o < kPlanOrders; ++o) {
             LinePlan qx{}, qy{}, qz{}, rx{}, ry{}, rz{};
-            if (!make_plan(Nx, qx, false, o) || !make_plan(Ny, qy, false, o) || !make_plan(Nz, qz, false, o)) continue;
+            if (!make_plan(Nx, qx, o) || !make_plan(Ny, qy, o) || !make_plan(Nz, qz, o)) continue;
             bool dup = false;
             for (int o2 = 0; o2 < o && !dup; ++o2)
-                if (make_plan(Nx, rx, false, o2) && make_plan(Ny, ry, false, o2) && make_plan(Nz, rz, false, o2))
+                if (make_plan(Nx, rx, o2) && make_plan(Ny, ry, o2) && make_plan(Nz, rz, o2))
                     dup = same(qx, rx) && same(qy, ry) && same(qz, rz);
             if (!dup) cand.push_back(m3d_tune{0, 0, G0, Y0, X0, 0, 0, 0, o});
         }
@@ -2361,9 +2365,9 @@ int m3d_solver::autotune(int sweeps, m3d_tune* out) {
         use_fast = c.fast != 0;
         use_tma_y = c.tma_y != 0;
         use_slab = c.slab != 0;
-        make_plan(Nx, px, false, c.schedule);
-        make_plan(Ny, py, false, c.schedule);
-        make_plan(Nz, pz, false, c.schedule);
+        make_plan(Nx, px, c.schedule);
+        make_plan(Ny, py, c.schedule);
+        make_plan(Nz, pz, c.schedule);
         (fp64 ? G64 : G32) = c.G;
         (fp64 ? TZy64 : TZy32) = c.tzy;
         (fp64 ? TZx64 : TZx32) = c.tzx;
@@ -2415,9 +2419,9 @@ int m3d_autotune(m3d_solver* h, int sweeps, m3d_tune* out) {
     h->use_fast = t.fast != 0;
     h->use_tma_y = t.tma_y != 0;
     h->use_slab = t.slab != 0;
-    make_plan(h->Nx, h->px, false, t.schedule);
-    make_plan(h->Ny, h->py, false, t.schedule);
-    make_plan(h->Nz, h->pz, false, t.schedule);
+    make_plan(h->Nx, h->px, t.schedule);
+    make_plan(h->Ny, h->py, t.schedule);
+    make_plan(h->Nz, h->pz, t.schedule);
     (fp64 ? h->G64 : h->G32) = t.G;
     (fp64 ? h->TZy64 : h->TZy32) = t.tzy;
     (fp64 ? h->TZx64 : h->TZx32) = t.tzx;

@@ -92,7 +92,7 @@ __device__ __forceinline__ void cp_wait_all() { asm volatile("cp.async.wait_grou
 // is then fetched after the previous one is stored)
 template <int MaxR>
 __global__ void __launch_bounds__(256) k2d_rows(double2* __restrict__ buf, double2* __restrict__ eps, const double2* __restrict__ twy,
-                         LinePlan py, int G, int nlines, int sign, long long xy, int nbuf) {
+                         const __grid_constant__ LinePlan py, int G, int nlines, int sign, long long xy, int nbuf) {
     extern __shared__ __align__(16) char smem_raw[];
     const int Ny = py.n;
     const int tsz = G * Ny;
@@ -149,17 +149,17 @@ __global__ void __launch_bounds__(256) k2d_rows(double2* __restrict__ buf, doubl
 // Column turnaround: TZ consecutive columns y of all Nx rows and 3 components;
 // forward FFT along x, -Gamma0 : tau^ per mode (k = 0 -> E * xy), inverse FFT.
 template <int MaxR>
-__global__ void __launch_bounds__(256) k2d_cols(double2* __restrict__ buf, const double2* __restrict__ twx, LinePlan px, int Ny, int TZ,
+__global__ void __launch_bounds__(256) k2d_cols(double2* __restrict__ buf, const double2* __restrict__ twx, const __grid_constant__ LinePlan px, int Ny, FastDiv dTZ,
                          Consts2D k, long long xy) {
     extern __shared__ __align__(16) char smem_raw[];
-    const int Nx = px.n;
+    const int Nx = px.n, TZ = dTZ.d;
     double2* tw = (double2*)smem_raw;
     double2* A = tw + Nx;  // [c][x][tz]
     double2* B = A + (size_t)3 * Nx * TZ;
     const int y0 = blockIdx.x * TZ;
     for (int i = threadIdx.x; i < Nx; i += blockDim.x) tw[i] = twx[i];
     for (int i = threadIdx.x; i < 3 * Nx * TZ; i += blockDim.x) {
-        const int tz = i % TZ, cx = i / TZ, x = cx % Nx, c = cx / Nx;
+        const int cx = dTZ.div(i), tz = i - cx * TZ, c = px.dn.div(cx), x = cx - c * Nx;
         const int y = y0 + tz;
         A[i] = y < Ny ? buf[c * xy + (long long)x * Ny + y] : make_double2(0, 0);
     }
@@ -169,7 +169,7 @@ __global__ void __launch_bounds__(256) k2d_cols(double2* __restrict__ buf, const
     double2* o = (r == A) ? B : A;
     // Green operator (setGF :49-103, multiplyGF :105-138)
     for (int i = threadIdx.x; i < Nx * TZ; i += blockDim.x) {
-        const int tz = i % TZ, x = i / TZ, y = y0 + tz;
+        const int x = dTZ.div(i), tz = i - x * TZ, y = y0 + tz;
         double2 t[3];
 #pragma unroll
         for (int c = 0; c < 3; ++c) t[c] = r[(c * Nx + x) * TZ + tz];
@@ -202,7 +202,7 @@ __global__ void __launch_bounds__(256) k2d_cols(double2* __restrict__ buf, const
     __syncthreads();
     double2* s = fft_lines<double2, MaxR>(o, r, tw, px, L, +1);
     for (int i = threadIdx.x; i < 3 * Nx * TZ; i += blockDim.x) {
-        const int tz = i % TZ, cx = i / TZ, x = cx % Nx, c = cx / Nx;
+        const int cx = dTZ.div(i), tz = i - cx * TZ, c = px.dn.div(cx), x = cx - c * Nx;
         const int y = y0 + tz;
         if (y < Ny) buf[c * xy + (long long)x * Ny + y] = s[i];
     }
@@ -299,7 +299,7 @@ struct m3d_solver2d {
             k2d_rows<decltype(r)::value><<<rows_grid, 256, rows_smem(), stream>>>(buf, nullptr, twy, py, G, nlines, -1, xy, rows_nbuf);
         });
         with_radix(px, [&](auto r) {
-            k2d_cols<decltype(r)::value><<<(Ny + TZ - 1) / TZ, 256, cols_smem(), stream>>>(buf, twx, px, Ny, TZ, k, xy);
+            k2d_cols<decltype(r)::value><<<(Ny + TZ - 1) / TZ, 256, cols_smem(), stream>>>(buf, twx, px, Ny, fast_div(TZ), k, xy);
         });
         with_radix(py, [&](auto r) {
             k2d_rows<decltype(r)::value><<<rows_grid, 256, rows_smem(), stream>>>(buf, eps, twy, py, G, nlines, +1, xy, rows_nbuf);
