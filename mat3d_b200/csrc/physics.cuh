@@ -641,14 +641,30 @@ __host__ __device__ inline double refine_inner_tol(double tol, double res) {
     return fmin(0.1, fmax(2e-5, need));
 }
 
+// Loop control of a graph-captured solve, folded into the finalize: the while
+// node's condition stays set until the last iterating entry is done (a kernel of
+// its own at the end of every trip cost 2-4 us a sweep).  Every entry stops by its
+// own rule or at its iteration cap, so the loop ends.
+struct LoopEnd {
+    cudaGraphConditionalHandle h = 0;
+    int* ndone = nullptr;  // entries done so far (null: no loop to control)
+    int total = 0;
+    __device__ __forceinline__ void entry_done(const Ctl& c) const {
+        if (ndone && c.done && atomicAdd(ndone, 1) + 1 == total) cudaGraphSetConditional(h, 0u);
+    }
+};
+
 static __global__ void k_finalize(Ctl* ctl, const double* __restrict__ partials, int NS, int nblk, int policy, double V,
-                                  const Ctl* outer) {
+                                  const Ctl* outer, LoopEnd loop) {
     const int b = blockIdx.x;
     if (ctl[b].done) return;
     __shared__ double red[256];
     __shared__ double tot[16];
     sum_partials(partials, NS, nblk, b, red, tot);
-    if (threadIdx.x == 0) policy_linear(ctl[b], tot, policy, V, outer, b);
+    if (threadIdx.x == 0) {
+        policy_linear(ctl[b], tot, policy, V, outer, b);
+        loop.entry_done(ctl[b]);
+    }
 }
 
 // Finalize run by the last block of the pass that produced the partials.
@@ -657,12 +673,14 @@ struct FinLinear {
     double V;
     const Ctl* outer;
     int* counter;
+    LoopEnd loop{};
     __device__ __forceinline__ void run(Ctl* ctl, const double* partials, int NS, int nblk, int b, double* red,
                                         double* tot) const {
         sum_partials(partials, NS, nblk, b, red, tot);
         if (threadIdx.x == 0) {
             if (NS < 2) tot[1] = 0;  // the residual policies use tot[0] only
             policy_linear(ctl[b], tot, policy, V, outer, b);
+            loop.entry_done(ctl[b]);
         }
     }
 };

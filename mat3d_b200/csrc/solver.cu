@@ -287,6 +287,7 @@ struct m3d_solver {
     template <typename T, int CC, class Spec> int pass_x(Spec op, Ctl* ctl, typename Cx<T>::t* sp);
     template <typename T, int CC, class Epi, class Fin> int pass_zinv(Epi epi, Ctl* ctl, typename Cx<T>::t* sp, Fin fin);
     int* d_counter = nullptr;  // completion counters of the fused finalize, one per batch entry
+    LoopEnd loop_end{};        // of the while node whose body is being captured (none outside a capture)
     // TMA-staged y pass: tensor maps of the half spectrum viewed as rows of
     // 2*Hzp FP32 / FP64 scalars (built for the current buffer and batch)
     bool use_tma_y = false;
@@ -333,8 +334,8 @@ struct m3d_solver {
     template <int CC>
     int run_refine(double tol_field, int max_iter);
     // Graph-captured solves: the whole iteration runs as one CUDA graph launch,
-    // its loops as conditional while nodes that a one-block kernel re-arms
-    // after each sweep (no host round trip until the batch is done).
+    // its loops as conditional while nodes that the finalize of the last
+    // iterating entry ends (no host round trip until the batch is done).
     bool use_graph = true;
     // Compacted sweeps (multi-entry graph solves, residual rule): the loop
     // runs as a chain of while nodes over shrinking launch grids (B, B/2,
@@ -363,7 +364,8 @@ struct m3d_solver {
         long long key = -1;
     };
     GraphSlot gslot[3];  // 0: linear residual rule, 1: linear reference rule, 2: refinement
-    int* d_trips = nullptr;  // [0] loop trips this run, [1] outer trips total, [2] inner trips this round, [3] inner total
+    int* d_trips = nullptr;  // [0] loop trips this run, [1] outer trips total, [2] inner trips this round, [3] inner total,
+                             // [4] linear and [5] inner entries done (LoopEnd)
     unsigned long long* d_pstat = nullptr;  // phase-map statistics: [0, 16) counts per id, [16] id sum, [17] first bad voxel
     int load_phase(int r, const int32_t* phase, int nph, std::vector<long long>& counts, long long& idsum,
                    long long& bad);
@@ -839,7 +841,7 @@ int m3d_solver::launch_sweep(Pro pro, Spec spec, Epi epi, Ctl* ctl, typename Cx<
     prof_pass(3);
     pass_y<T>(+1, CC, ctl, sp);
     prof_pass(4);
-    pass_zinv<T, CC>(epi, ctl, sp, FinLinear{policy, (double)g.V, outer, d_counter});
+    pass_zinv<T, CC>(epi, ctl, sp, FinLinear{policy, (double)g.V, outer, d_counter, loop_end});
     prof_pass(5);
     M3D_CUDA(cudaGetLastError());
     return M3D_OK;
@@ -854,7 +856,7 @@ int m3d_solver::launch_check(Ctl* ctl, const void* x, typename Cx<T>::t* sp) {
     pass_zfwd<T, CC>(pro, ctl, sp);
     pass_y<T>(-1, CC, ctl, sp);
     const int xblk = pass_x<T, CC>(sv, ctl, sp);
-    k_finalize<<<B, 256, 0, stream>>>(ctl, d_part, 2, xblk, POL_REF_CHECK, (double)g.V, nullptr);
+    k_finalize<<<B, 256, 0, stream>>>(ctl, d_part, 2, xblk, POL_REF_CHECK, (double)g.V, nullptr, loop_end);
     st.kernel_launches += 1;
     M3D_CUDA(cudaGetLastError());
     return M3D_OK;
@@ -954,7 +956,7 @@ int m3d_solver::launch_em_slab(Ctl* ctl, T* x, const float* r, typename Cx<T>::t
     if (!plane) pass_x<T, CC>(green<T, CC>(zero_k0), ctl, sp);
     prof_pass(3);
     prof_pass(4);
-    const int rc = pass_slab<T, CC, true>(ctl, x, r, sp, FinLinear{policy, (double)g.V, outer, d_counter});
+    const int rc = pass_slab<T, CC, true>(ctl, x, r, sp, FinLinear{policy, (double)g.V, outer, d_counter, loop_end});
     prof_pass(5);
     return rc;
 }
@@ -1114,20 +1116,6 @@ int m3d_solver::run_refine(double tol_field, int max_iter) {
 }
 
 // ---- graph-captured solves -------------------------------------------------------
-// Loop control of a captured while node: continue while any entry of the batch
-// is not done.  Every entry stops by its own rule or at its iteration cap; the
-// trip count is a second cap on the loop itself.
-__global__ void k_loop_cond(cudaGraphConditionalHandle h, const Ctl* __restrict__ ctl, int B, int* trips, int slot) {
-    int any = 0;
-    for (int b = threadIdx.x; b < B; b += blockDim.x) any |= (ctl[b].done == 0);
-    any = __syncthreads_or(any);
-    if (threadIdx.x == 0) {
-        const int t = ++trips[slot];
-        ++trips[slot + 1];
-        cudaGraphSetConditional(h, (any && t <= ctl[0].max_iter + 2) ? 1u : 0u);
-    }
-}
-
 // One block rebuilds the live list from the control blocks: live[0] = the
 // number of entries not done, live[1..] their ids in increasing order.
 __device__ void build_live(const Ctl* __restrict__ ctl, int B, int* live) {
@@ -1185,11 +1173,16 @@ __global__ void k_loop_cond_live(cudaGraphConditionalHandle h, const Ctl* __rest
 // every entry a fresh inner control block (the entries already converged stay
 // done) and arm both loops.
 __global__ void k_refine_mid(cudaGraphConditionalHandle h_outer, cudaGraphConditionalHandle h_inner, Ctl* ctl,
-                             Ctl* ctl_in, int B, int* trips) {
+                             Ctl* ctl_in, int B, int* trips, int one_loop) {
+    __shared__ int most, ndone;  // sweeps of the previous round's longest entry; entries already converged
+    if (threadIdx.x == 0) most = ndone = 0;
+    __syncthreads();
     int any = 0;
     for (int b = threadIdx.x; b < B; b += blockDim.x) {
         Ctl& o = ctl[b];
         o.aux[1] += (double)ctl_in[b].iters;
+        atomicMax(&most, ctl_in[b].iters);
+        if (o.done) atomicAdd(&ndone, 1);
         Ctl c;
         memset(&c, 0, sizeof(c));
         c.gkind = o.gkind; c.gnyq = o.gnyq; c.gxw = o.gxw; c.gp1 = o.gp1; c.gp2 = o.gp2;
@@ -1204,6 +1197,8 @@ __global__ void k_refine_mid(cudaGraphConditionalHandle h_outer, cudaGraphCondit
         const int t = ++trips[0];
         ++trips[1];
         trips[2] = 0;
+        if (one_loop) trips[3] += most;
+        trips[5] = ndone;
         const unsigned go = (any && t <= ctl[0].max_iter + 2) ? 1u : 0u;
         cudaGraphSetConditional(h_outer, go);
         cudaGraphSetConditional(h_inner, go);
@@ -1335,6 +1330,8 @@ int m3d_solver::run_linear_graph(double tol_field, double tol_eq, int criterion,
             M3D_CAP(cudaGraphConditionalHandleCreate(&h, top, 1, cudaGraphCondAssignDefault));
             M3D_CAP(add_while(top, nullptr, 0, h, &node, &body));
             M3D_CAP(cudaStreamBeginCaptureToGraph(stream, body, nullptr, nullptr, 0, cudaStreamCaptureModeRelaxed));
+            // the finalize of a sweep (under the reference rule: of its check pass) ends the loop
+            loop_end = LoopEnd{h, d_trips + 4, B};
             if (slab) {
                 rc = launch_em_slab<T, CC>(d_ctl, x, nullptr, sp, 0, POL_RESIDUAL, nullptr);
             } else if (resid) {
@@ -1343,9 +1340,8 @@ int m3d_solver::run_linear_graph(double tol_field, double tol_eq, int criterion,
                 rc = launch_em<T, CC>(d_ctl, x, nullptr, sp, 0, POL_REF_SWEEP, nullptr);
                 if (!rc) rc = launch_check<T, CC>(d_ctl, x, sp);
             }
+            loop_end = LoopEnd{};
             if (rc) M3D_CAP(cudaErrorUnknown);
-            k_loop_cond<<<1, 256, 0, stream>>>(h, d_ctl, B, d_trips, 0);
-            M3D_CAP(cudaGetLastError());
             M3D_CAP(cudaStreamEndCapture(stream, &got));
         }
         st.kernel_launches = kl;
@@ -1359,7 +1355,9 @@ int m3d_solver::run_linear_graph(double tol_field, double tol_eq, int criterion,
     if (rc) return rc;
     int trips[8];
     M3D_CUDA(cudaMemcpy(trips, d_trips, sizeof(trips), cudaMemcpyDeviceToHost));
-    st.kernel_launches += 1 + (long long)lv.size() + (long long)trips[0] * (slab ? 3 : (resid ? 6 : 10));
+    // launches per trip: the passes, of a compacted loop one more
+    const int ntrips = lv.empty() ? max_iters() : trips[0];
+    st.kernel_launches += 1 + (long long)lv.size() + (long long)ntrips * ((slab ? 2 : (resid ? 5 : 9)) + (lv.empty() ? 0 : 1));
     long long sw = 0;
     int status = M3D_OK;
     for (int b = 0; b < B; ++b) {
@@ -1416,7 +1414,7 @@ int m3d_solver::run_refine_graph(double tol_field, int max_iter) {
         EpiDefect<CC> epi = tab(EpiDefect<CC>{d_phase, x, d_r32, g.V, dm(off_Os), nph_max(), nullptr});
         rc = launch_sweep<double, CC>(pro, green<double, CC>(0), epi, d_ctl, sp64, POL_REFINE_OUTER, nullptr);
         if (rc) M3D_CAP(cudaErrorUnknown);
-        k_refine_mid<<<1, 256, 0, stream>>>(h_out, h_in, d_ctl, d_ctl_in, B, d_trips);
+        k_refine_mid<<<1, 256, 0, stream>>>(h_out, h_in, d_ctl, d_ctl_in, B, d_trips, lv.empty() ? 1 : 0);
         M3D_CAP(cudaGetLastError());
         M3D_CAP(cudaMemsetAsync(d_delta, 0, dbytes, stream));
         // two-pass sweeps: the correction starts at 0, whose spectrum is 0
@@ -1452,10 +1450,11 @@ int m3d_solver::run_refine_graph(double tol_field, int max_iter) {
                 k_loop_cond_live<<<1, 256, 0, stream>>>(hs[k], d_ctl_in, B, d_live,
                                                         k + 1 < lv.size() ? lv[k + 1] : 0, d_trips, 2);
             } else {
+                loop_end = LoopEnd{hs[k], d_trips + 5, B};
                 rc = slab ? launch_em_slab<float, CC>(d_ctl_in, d_delta, d_r32, sp32, 1, POL_REFINE_INNER, d_ctl)
                           : launch_em<float, CC>(d_ctl_in, d_delta, d_r32, sp32, 1, POL_REFINE_INNER, d_ctl);
+                loop_end = LoopEnd{};
                 if (rc) M3D_CAP(cudaErrorUnknown);
-                k_loop_cond<<<1, 256, 0, stream>>>(hs[k], d_ctl_in, B, d_trips, 2);
             }
             M3D_CAP(cudaGetLastError());
             M3D_CAP(cudaStreamEndCapture(stream, &got));
@@ -1471,7 +1470,7 @@ int m3d_solver::run_refine_graph(double tol_field, int max_iter) {
     if (rc) return rc;
     int trips[8];
     M3D_CUDA(cudaMemcpy(trips, d_trips, sizeof(trips), cudaMemcpyDeviceToHost));
-    st.kernel_launches += 1 + (long long)trips[1] * (6 + (long long)lv.size()) + (long long)trips[3] * (slab ? 3 : 6);
+    st.kernel_launches += 1 + (long long)trips[1] * (6 + (long long)lv.size()) + (long long)trips[3] * ((slab ? 2 : 5) + (lv.empty() ? 0 : 1));
     long long n64 = 0, n32 = 0;
     int status = M3D_OK;
     for (int b = 0; b < B; ++b) {
@@ -2057,12 +2056,17 @@ int m3d_run(m3d_solver* h, double tol_field, double tol_eq, int nInc, int criter
 
 }  // extern "C"
 
-static int assemble_rve(m3d_solver* h, int r, double* Ceff, double* Seff, double* ep_means, double* sig_means);
+static int assemble_rve(m3d_solver* h, int r, const double* sums, double* Ceff, double* Seff, double* ep_means,
+                        double* sig_means);
 
-// means of the strain-like and stress-like fields of entry b
+// Sums of the state and of the other field (O x) of entries b0 + blockIdx.y:
+// per-block partials part[(entry * 2C + k) * gridDim.x + block].
 template <typename TX, int CC>
 __global__ void k_means(const TX* __restrict__ x, const uint8_t* __restrict__ phase, const double* __restrict__ mats,
-                        int b, long long V, double* __restrict__ part) {
+                        int b0, int lc, long long mstride, long long V, double* __restrict__ part) {
+    const int b = b0 + blockIdx.y, r = b / lc;
+    phase += (long long)r * V;
+    mats += (long long)r * mstride;
     double acc[2 * CC] = {};
     for (long long v = blockIdx.x * (long long)blockDim.x + threadIdx.x; v < V; v += (long long)gridDim.x * blockDim.x) {
         double xv[CC];
@@ -2079,7 +2083,53 @@ __global__ void k_means(const TX* __restrict__ x, const uint8_t* __restrict__ ph
         }
     }
     __shared__ double red[32 * 2 * CC];
-    block_reduce_store<2 * CC>(acc, red, part, 0, gridDim.x, blockIdx.x);
+    block_reduce_store<2 * CC>(acc, red, part, blockIdx.y, gridDim.x, blockIdx.x);
+}
+// their totals, out[entry * NS + k], in a fixed order
+static __global__ void k_means_sum(const double* __restrict__ part, int NS, int nblk, double* __restrict__ out) {
+    __shared__ double red[256];
+    __shared__ double tot[16];
+    sum_partials(part, NS, nblk, blockIdx.x, red, tot);
+    if (threadIdx.x < NS) out[blockIdx.x * NS + threadIdx.x] = tot[threadIdx.x];
+}
+
+// Sums of entries b0 .. b0 + nb - 1 (2C each: the state, the other field): two
+// launches and one copy for all of them.  (A launch, a copy and a host sum per
+// entry took 30 us each, 4.4 of 21 ms of a homogenization of 24 RVEs at 32^3.)
+static int entry_sums(m3d_solver* h, int b0, int nb, double* sums) {
+    const int C = h->C, nblk = 296;
+    double* part = h->d_part;
+    double* tot = part + (size_t)nb * 2 * C * nblk;
+    if (h->part_cap < (size_t)nb * 2 * C * (nblk + 1)) return fail(M3D_ERR_STATE, "partials buffer too small");
+    const double* O = h->d_mats + h->off_O;
+    const int lc = h->entries_per_rve();
+    const dim3 grid(nblk, nb);
+    auto go = [&](auto x, auto cc) {
+        typedef typename std::remove_const<typename std::remove_pointer<decltype(x)>::type>::type TX;
+        k_means<TX, decltype(cc)::value><<<grid, 256, 0, h->stream>>>(x, h->d_phase, O, b0, lc, h->mstride, h->g.V, part);
+    };
+    const bool f32 = h->prec == M3D_PREC_FP32;
+    if (C == 6) { if (f32) go((const float*)h->d_x, IntC<6>{}); else go((const double*)h->d_x, IntC<6>{}); }
+    else { if (f32) go((const float*)h->d_x, IntC<3>{}); else go((const double*)h->d_x, IntC<3>{}); }
+    M3D_CUDA(cudaGetLastError());
+    k_means_sum<<<nb, 256, 0, h->stream>>>(part, 2 * C, nblk, tot);
+    M3D_CUDA(cudaGetLastError());
+    h->st.kernel_launches += 2;
+    M3D_CUDA(cudaMemcpyAsync(sums, tot, (size_t)nb * 2 * C * sizeof(double), cudaMemcpyDeviceToHost, h->stream));
+    M3D_CUDA(cudaStreamSynchronize(h->stream));
+    return M3D_OK;
+}
+// volume averages of one entry from its sums: the state is strain-like in the
+// primal scheme, stress-like in the dual one
+static void sums_to_means(const m3d_solver* h, int r, const double* s, double* strain_mean, double* stress_mean) {
+    const double V = (double)h->g.V;
+    const bool primal = h->rv[r].scheme == 1;
+    double* prim = primal ? strain_mean : stress_mean;
+    double* dual = primal ? stress_mean : strain_mean;
+    for (int c = 0; c < h->C; ++c) {
+        if (prim) prim[c] = s[c] / V;
+        if (dual) dual[c] = s[h->C + c] / V;
+    }
 }
 
 extern "C" {
@@ -2088,39 +2138,12 @@ int m3d_get_means(m3d_solver* h, int b, double* strain_mean, double* stress_mean
     if (!h) return fail(M3D_ERR_ARG, "NULL handle");
     if (!h->run_done) return fail(M3D_ERR_STATE, "no finished run");
     if (b < 0 || b >= h->B) return fail(M3D_ERR_ARG, "batch index out of range");
-    const int C = h->C;
     if (h->kind == M3D_KIND_MECH && h->behav != M3D_BEHAV_ELASTIC)
         return h->in.means(h, b, strain_mean, stress_mean);
-    const int nblk = 296;
-    double* part = h->d_part;
-    if (h->part_cap < (size_t)nblk * 2 * C) return fail(M3D_ERR_STATE, "partials buffer too small");
-    const int r = h->rve_of(b);
-    const double* O = h->d_mats + (size_t)r * h->mstride + h->off_O;
-    const uint8_t* ph = h->d_phase + (size_t)r * h->g.V;
-    if (C == 6) {
-        if (h->prec == M3D_PREC_FP32) k_means<float, 6><<<nblk, 256, 0, h->stream>>>((const float*)h->d_x, ph, O, b, h->g.V, part);
-        else k_means<double, 6><<<nblk, 256, 0, h->stream>>>((const double*)h->d_x, ph, O, b, h->g.V, part);
-    } else {
-        if (h->prec == M3D_PREC_FP32) k_means<float, 3><<<nblk, 256, 0, h->stream>>>((const float*)h->d_x, ph, O, b, h->g.V, part);
-        else k_means<double, 3><<<nblk, 256, 0, h->stream>>>((const double*)h->d_x, ph, O, b, h->g.V, part);
-    }
-    h->st.kernel_launches += 1;
-    M3D_CUDA(cudaGetLastError());
-    std::vector<double> hp((size_t)nblk * 2 * C);
-    M3D_CUDA(cudaMemcpyAsync(hp.data(), part, hp.size() * sizeof(double), cudaMemcpyDeviceToHost, h->stream));
-    M3D_CUDA(cudaStreamSynchronize(h->stream));
     double s[12] = {};
-    for (int k = 0; k < 2 * C; ++k)
-        for (int i = 0; i < nblk; ++i) s[k] += hp[(size_t)k * nblk + i];
-    const double V = (double)h->g.V;
-    // state = strain-like in the primal scheme, stress-like in the dual scheme
-    const bool primal = h->rv[r].scheme == 1;
-    double* prim = primal ? strain_mean : stress_mean;
-    double* dual = primal ? stress_mean : strain_mean;
-    for (int c = 0; c < C; ++c) {
-        if (prim) prim[c] = s[c] / V;
-        if (dual) dual[c] = s[C + c] / V;
-    }
+    const int rc = entry_sums(h, b, 1, s);
+    if (rc) return rc;
+    sums_to_means(h, h->rve_of(b), s, strain_mean, stress_mean);
     return M3D_OK;
 }
 
@@ -2150,8 +2173,11 @@ int m3d_homogenize(m3d_solver* h, double tol_field, double tol_eq, int criterion
     if (rc != M3D_OK && rc != M3D_NOT_CONVERGED) return rc;
     const int status = rc;
     h->run_done = true;
+    std::vector<double> sums((size_t)R * C * 2 * C);
+    rc = entry_sums(h, 0, R * C, sums.data());
+    if (rc) return rc;
     for (int r = 0; r < R; ++r) {
-        rc = assemble_rve(h, r, Ceff ? Ceff + (size_t)r * C * C : nullptr, Seff ? Seff + (size_t)r * C * C : nullptr,
+        rc = assemble_rve(h, r, &sums[(size_t)r * C * 2 * C], Ceff ? Ceff + (size_t)r * C * C : nullptr, Seff ? Seff + (size_t)r * C * C : nullptr,
                           ep_means ? ep_means + (size_t)r * C * C : nullptr,
                           sig_means ? sig_means + (size_t)r * C * C : nullptr);
         if (rc) return rc;
@@ -2164,15 +2190,12 @@ int m3d_homogenize(m3d_solver* h, double tol_field, double tol_eq, int criterion
 }  // extern "C"
 
 // Effective tensor of RVE r from the means of its C load-case entries.
-static int assemble_rve(m3d_solver* h, int r, double* Ceff, double* Seff, double* ep_means, double* sig_means) {
+static int assemble_rve(m3d_solver* h, int r, const double* sums, double* Ceff, double* Seff, double* ep_means,
+                        double* sig_means) {
     const int C = h->C;
-    int rc;
     // strain-like means g[w][c], stress-like q[w][c] per load case w
     std::vector<double> gm(C * C), qm(C * C);
-    for (int w = 0; w < C; ++w) {
-        rc = m3d_get_means(h, r * C + w, &gm[w * C], &qm[w * C]);
-        if (rc) return rc;
-    }
+    for (int w = 0; w < C; ++w) sums_to_means(h, r, sums + (size_t)w * 2 * C, &gm[w * C], &qm[w * C]);
     // Assembly exactly as the reference: one matrix stores the means with one
     // ROW per load case, the other with one COLUMN per load case, and the
     // result is X = first^-1 * second.
