@@ -98,8 +98,9 @@ typedef struct {
     double k0;               /* reference conductivity (thermal) */
     double vol_fraction[16]; /* per phase id */
     long long kernel_launches; /* kernels this handle launched since creation */
-    int passes_per_sweep;    /* launches per linear sweep of the last run: 5 (z, y, x, y, z passes) or
-                                2 (x turnaround + the y-z slab pass, per-component operators) */
+    int passes_per_sweep;    /* launches per linear sweep of the last run: 5 (z, y, x, y, z passes),
+                                4 (the z passes fused with the next sweep's) or 2 (x turnaround + the
+                                y-z slab pass, or kz-plane pass + fused z pass) */
 } m3d_stats;
 
 /* Create a solver for an Nx x Ny x Nz grid.  `batch` independent solves
@@ -181,7 +182,9 @@ typedef struct {
     /* the same time split by pass (events around each pass of the linear
        sweeps): z forward, y forward, x turnaround, y inverse, z inverse; on
        two-pass sweeps (m3d_stats.passes_per_sweep == 2) slot 2 holds the x
-       turnaround and slot 4 the y-z slab pass, slots 0, 1 and 3 stay 0 */
+       turnaround (kz-plane pass) and slot 4 the y-z slab (fused z) pass, slots
+       0, 1 and 3 stay 0; where the z passes are fused slot 4 holds the fused
+       pass and slot 0 stays 0 */
     double pass_ms_fp64[5];
     double pass_ms_fp32[5];
 } m3d_profile;
@@ -329,7 +332,7 @@ typedef struct {
     int G, tzy, tzx;  /* generic kernels: z lines per CTA, y / x tile columns */
     double sweep_us;  /* measured time of one sweep with this schedule */
     int candidates;   /* schedules timed */
-    int slab;         /* 1: two-pass sweeps (x turnaround + y-z slab pass) */
+    int slab;         /* 1: sweeps whose last kernel also does the next z forward (two or four passes) */
     int schedule;     /* generic line FFTs: order of the radix stages (0 largest odd factor first,
                          1 smallest odd first, 2 powers of two first, 3 radix-4 for the powers of two) */
 } m3d_tune;

@@ -1,7 +1,8 @@
 // generic_r13.cu -- the generic passes with compile-time butterflies up to
-// radix 13 (generic_launch.cuh).
-#include "generic_launch.cuh"
+// radix 13 (generic_launch.cuh, zmid_launch.cuh).
+#include "zmid_launch.cuh"
 
 namespace m3d {
 M3D_GEN_ALL(, 13)
+M3D_GEN_ZMID_ALL(, 13)
 }  // namespace m3d

@@ -262,8 +262,8 @@ extern "C" int m3d_thermal_solve_noalloc(int Nx, int Ny, int Nz, double km, doub
 
     const size_t extra = 2 * (C * C + C) * sizeof(double) + 64;
     const size_t zsmem = (size_t)Nz * sizeof(double2) + 2 * (size_t)(G / 2) * C * Nz * sizeof(double2) + 16 + 32 * 32 * 8 + extra;
-    const size_t ysmem = (size_t)Ny * sizeof(double2) + 2 * (size_t)Ny * TZy * sizeof(double2);
-    const size_t xsmem = (size_t)Nx * sizeof(double2) + 2 * (size_t)C * Nx * TZx * sizeof(double2) + 16 + 32 * 32 * 8;
+    const size_t ysmem = col_tile_smem<double2>(Ny, TZy);
+    const size_t xsmem = col_tile_smem<double2>(Nx, C * TZx) + 16 + 32 * 32 * 8;
     const int ntzy = (g.Hzp + TZy - 1) / TZy, ntzx = (g.Hzp + TZx - 1) / TZx;
     const FastDiv dTZy = fast_div(TZy), dTZx = fast_div(TZx), dntzy = fast_div(ntzy), dntzx = fast_div(ntzx);
     {

@@ -125,6 +125,59 @@ __device__ __forceinline__ char* align_up(char* p, int a) {
     return (char*)(((uintptr_t)p + (a - 1)) & ~(uintptr_t)(a - 1));
 }
 
+// 8- or 16-byte asynchronous global->shared copy; src_bytes = 0 writes zeros
+__device__ __forceinline__ void cp_async(void* smem_dst, const void* gmem_src, int bytes, int src_bytes) {
+    const unsigned d = (unsigned)__cvta_generic_to_shared(smem_dst);
+    if (bytes == 8)
+        asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;\n" ::"r"(d), "l"(gmem_src), "r"(src_bytes));
+    else
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(d), "l"(gmem_src), "r"(src_bytes));
+}
+__device__ __forceinline__ void cp_async_wait_all() {
+    asm volatile("cp.async.commit_group;\n" ::);
+    asm volatile("cp.async.wait_group 0;\n" ::);
+}
+
+// Column tiles of the y and x passes: TZ consecutive modes of rows e of the half
+// spectrum, element (e, col) at e*TZ + col of the tile.  Two modes per 16-byte
+// copy where the tile width is even (FP32; rows and tiles start at even modes).
+template <typename C2, class Row>
+__device__ __forceinline__ void col_tile_load(C2* A, int n, const FastDiv& dTZ, int avail, Row row) {
+    const int TZ = dTZ.d;
+    if (sizeof(C2) == 8 && !(TZ & 1)) {
+        for (int i = 2 * threadIdx.x; i < n * TZ; i += 2 * blockDim.x) {
+            const int e = dTZ.div(i), col = i - e * TZ;
+            cp_async(A + i, row(e) + (col < avail ? col : 0), 16, col < avail ? 16 : 0);
+        }
+    } else {
+        for (int i = threadIdx.x; i < n * TZ; i += blockDim.x) {
+            const int e = dTZ.div(i), col = i - e * TZ;
+            cp_async(A + i, row(e) + (col < avail ? col : 0), (int)sizeof(C2), col < avail ? (int)sizeof(C2) : 0);
+        }
+    }
+    cp_async_wait_all();
+}
+template <typename C2, class Row>
+__device__ __forceinline__ void col_tile_store(const C2* R, int n, const FastDiv& dTZ, int avail, Row row) {
+    const int TZ = dTZ.d;
+    if (sizeof(C2) == 8 && !(TZ & 1)) {
+        for (int i = 2 * threadIdx.x; i < n * TZ; i += 2 * blockDim.x) {
+            const int e = dTZ.div(i), col = i - e * TZ;
+            if (col < avail) *reinterpret_cast<float4*>(row(e) + col) = *reinterpret_cast<const float4*>(R + i);
+        }
+    } else {
+        for (int i = threadIdx.x; i < n * TZ; i += blockDim.x) {
+            const int e = dTZ.div(i), col = i - e * TZ;
+            if (col < avail) row(e)[col] = R[i];
+        }
+    }
+}
+// shared memory of a column tile kernel: twiddles (an even number, so that the
+// tiles are 16-byte aligned) and two tiles
+template <typename C2> constexpr size_t col_tile_smem(int n, int lines) {
+    return (size_t)((n + 1) & ~1) * sizeof(C2) + 2 * (size_t)n * lines * sizeof(C2) + 16;
+}
+
 // ============================================================================
 // z forward: prologue (per voxel: C input values) -> pairs of real lines packed
 // as one complex line -> FFT along z -> split into two half spectra.
@@ -208,22 +261,17 @@ __global__ void __launch_bounds__(256) k_ypass(GridDims g, const __grid_constant
     extern __shared__ __align__(16) char smem_raw[];
     const int Ny = g.Ny, Hzp = g.Hzp, TZ = dTZ.d;
     C2* tw = (C2*)smem_raw;
-    C2* A = tw + Ny;
-    C2* B = A + (size_t)Ny * TZ;
+    C2* A = tw + ((Ny + 1) & ~1);
+    C2* B = A + (((size_t)Ny * TZ + 1) & ~(size_t)1);
     for (int i = threadIdx.x; i < Ny; i += blockDim.x) tw[i] = twy[i];
     const int x = dntz.div(blockIdx.x), kz0 = (blockIdx.x - x * dntz.d) * TZ;
     C2* base = spec + ((long long)cb * g.NL + (long long)x * Ny) * Hzp + kz0;
-    for (int i = threadIdx.x; i < Ny * TZ; i += blockDim.x) {
-        const int y = dTZ.div(i), col = i - y * TZ;
-        A[i] = (kz0 + col < Hzp) ? base[y * Hzp + col] : mk<C2>(0, 0);
-    }
+    auto row = [&](int y) { return base + y * Hzp; };
+    col_tile_load<C2>(A, Ny, dTZ, Hzp - kz0, row);
     __syncthreads();
     LineLayout L{TZ, TZ, 1, 0, TZ, true};
     C2* R = fft_lines<C2, MaxR>(A, B, tw, py, L, sign);
-    for (int i = threadIdx.x; i < Ny * TZ; i += blockDim.x) {
-        const int y = dTZ.div(i), col = i - y * TZ;
-        if (kz0 + col < Hzp) base[y * Hzp + col] = R[i];
-    }
+    col_tile_store<C2>(R, Ny, dTZ, Hzp - kz0, row);
 }
 
 // ============================================================================
@@ -242,17 +290,17 @@ __global__ void __launch_bounds__(256) k_xturn(GridDims g, const __grid_constant
     extern __shared__ __align__(16) char smem_raw[];
     const int Nx = g.Nx, Ny = g.Ny, Hzp = g.Hzp, TZ = dTZ.d;
     C2* tw = (C2*)smem_raw;
-    C2* A = tw + Nx;
-    C2* B = A + (size_t)C * Nx * TZ;
+    C2* A = tw + ((Nx + 1) & ~1);
+    C2* B = A + (((size_t)C * Nx * TZ + 1) & ~(size_t)1);
     double* red = (double*)align_up((char*)(B + (size_t)C * Nx * TZ), 16);
     for (int i = threadIdx.x; i < Nx; i += blockDim.x) tw[i] = twx[i];
     const int y = dntz.div(blockIdx.x), kz0 = (blockIdx.x - y * dntz.d) * TZ;
     C2* base = spec + ((long long)b * C * g.NL + y) * Hzp + kz0;
-    for (int i = threadIdx.x; i < C * Nx * TZ; i += blockDim.x) {
-        const int r = dTZ.div(i), col = i - r * TZ;
+    auto row = [&](int r) {
         const int c = px.dn.div(r), x = r - c * Nx;
-        A[i] = (kz0 + col < Hzp) ? base[((long long)c * g.NL + (long long)x * Ny) * Hzp + col] : mk<C2>(0, 0);
-    }
+        return base + ((long long)c * g.NL + (long long)x * Ny) * Hzp;
+    };
+    col_tile_load<C2>(A, C * Nx, dTZ, Hzp - kz0, row);
     __syncthreads();
     LineLayout L{C * TZ, TZ, 1, Nx * TZ, TZ, true};
     C2* R = fft_lines<C2, MaxR>(A, B, tw, px, L, -1);
@@ -278,11 +326,7 @@ __global__ void __launch_bounds__(256) k_xturn(GridDims g, const __grid_constant
     if constexpr (Spec::kInverse) {
         __syncthreads();
         C2* Q = fft_lines<C2, MaxR>(R, S, tw, px, L, +1);
-        for (int i = threadIdx.x; i < C * Nx * TZ; i += blockDim.x) {
-            const int r = dTZ.div(i), col = i - r * TZ;
-            const int c = px.dn.div(r), x = r - c * Nx;
-            if (kz0 + col < Hzp) base[((long long)c * g.NL + (long long)x * Ny) * Hzp + col] = Q[i];
-        }
+        col_tile_store<C2>(Q, C * Nx, dTZ, Hzp - kz0, row);
     }
 }
 

@@ -138,19 +138,6 @@ __global__ void __launch_bounds__(kFastThreads) k_ypass_fast(GridDims g, const t
 // ---------------------------------------------------------------------------
 // x turnaround
 // ---------------------------------------------------------------------------
-// 8- or 16-byte asynchronous global->shared copy; src_bytes = 0 writes zeros
-__device__ __forceinline__ void cp_async(void* smem_dst, const void* gmem_src, int bytes, int src_bytes) {
-    const unsigned d = (unsigned)__cvta_generic_to_shared(smem_dst);
-    if (bytes == 8)
-        asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;\n" ::"r"(d), "l"(gmem_src), "r"(src_bytes));
-    else
-        asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(d), "l"(gmem_src), "r"(src_bytes));
-}
-__device__ __forceinline__ void cp_async_wait_all() {
-    asm volatile("cp.async.commit_group;\n" ::);
-    asm volatile("cp.async.wait_group 0;\n" ::);
-}
-
 // warps per CTA of the x turnaround: as many as keep the staging <= 24 KB
 // (small CTAs: many resident per SM and a fine-grained tail)
 template <typename T, int N, int C>

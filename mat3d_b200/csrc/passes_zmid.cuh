@@ -9,7 +9,9 @@
 // FP32 256^3 2671 -> 967, FP32 64^3 64 -> 44.  Bound by latency: 12 warps per SM
 // of FP64 dependency chains (issue 24%, long scoreboard the largest stall); the
 // bytes of a J2 voxel (201 and its share of the spectrum) take 765 us at FP64
-// 256^3.
+// 256^3.  EM update, z forward + z inverse -> fused: FP32 thermal 256^3
+// 173 + 394 -> 212 us (124 us of bytes), FP64 thermal 128^3 52 + 76 -> 68, FP64
+// elastic 96^3 48 + 78 -> 54.
 //
 // CTAs of three warps walk tiles of G z lines of C components, C G/2 packed
 // complex lines (lines y, y + 1 of one component), LPW per warp.  The next
@@ -235,5 +237,96 @@ __global__ void __launch_bounds__(96, kZRowsMinB)
     block_reduce_store<Op::NSUM>(acc, red, partials, b, gridDim.x, blockIdx.x);
     fused_finalize(fin, ctl, partials, Op::NSUM, b);
 }
+
+// ---------------------------------------------------------------------------
+// The same for lengths without a compile-time transform (generic Stockham lines,
+// fft_smem.cuh): CTAs walk tiles of G lines of all components, packed line
+// p*C + c holding lines 2p, 2p + 1 of component c; one voxel per pointwise item.
+// Measured, elastic 75^3 FP32, six entries: z forward 63 + z inverse 108 us ->
+// 137.  Tiles as large as the separate passes' (48 KB): dealing a small grid to
+// at least four tiles per SM made most sizes slower (homogenization of eight
+// RVEs at 45^3 28.2 -> 36.9 ms).
+// ---------------------------------------------------------------------------
+template <typename T, int C, class Op, class Fin, int MaxR>
+__global__ void __launch_bounds__(256)
+    k_zmid_gen(GridDims g, const __grid_constant__ LinePlan pz, const typename Cx<T>::t* __restrict__ twz,
+               typename Cx<T>::t* __restrict__ spec, typename Op::Args args, Ctl* ctl, int G, double* partials, Fin fin) {
+    typedef typename Cx<T>::t C2;
+    const int b = entry_of(g, blockIdx.y);
+    if (b < 0 || ctl[b].done) return;
+    Op op;
+    op.a = args;
+    op.bind(b);
+    extern __shared__ __align__(16) char smem_raw[];
+    const int Nz = g.Nz, Hz = g.Hz, Hzp = g.Hzp;
+    const int nl = G / 2 * C;
+    C2* tw = (C2*)smem_raw;
+    C2* A = tw + Nz;
+    C2* B = A + (size_t)nl * Nz;
+    char* extra = align_up((char*)(B + (size_t)nl * Nz), 16);
+    double* red = (double*)extra;
+    for (int i = threadIdx.x; i < Nz; i += blockDim.x) tw[i] = twz[i];
+    op.load_smem(extra + 32 * Op::NSUM * sizeof(double), b);
+    const LineLayout L{nl, 1, 0, Nz, 1, false};
+    const T invV = (T)(1.0 / (double)g.V);
+    double acc[Op::NSUM] = {};
+    const int ntiles = (int)((g.NL + G - 1) / G);
+#pragma unroll 1
+    for (int ti = blockIdx.x; ti < ntiles; ti += gridDim.x) {
+        const long long l0 = (long long)ti * G;
+        for (int i = threadIdx.x; i < nl * Hz; i += blockDim.x) {
+            const int pc = g.dHz.div(i), k = i - pc * Hz;
+            const int p = pc / C, c = pc - p * C;
+            const long long la = l0 + 2 * p;
+            const C2* s = spec + (((long long)b * C + c) * g.NL + la) * Hzp + k;
+            const C2 a = la < g.NL ? s[0] : mk<C2>(0, 0);
+            const C2 q = la + 1 < g.NL ? s[Hzp] : mk<C2>(0, 0);
+            C2* line = A + (size_t)pc * Nz;
+            if (k == 0 || 2 * k == Nz) {
+                line[k] = mk<C2>(a.x, q.x);
+            } else {
+                line[k] = mk<C2>(a.x - q.y, a.y + q.x);
+                line[Nz - k] = mk<C2>(a.x + q.y, q.x - a.y);
+            }
+        }
+        __syncthreads();
+        C2* R = fft_lines<C2, MaxR>(A, B, tw, pz, L, +1);
+        C2* S = R == A ? B : A;
+        for (int i = threadIdx.x; i < G * Nz; i += blockDim.x) {
+            const int gi = pz.dn.div(i), z = i - gi * Nz;
+            const long long l = l0 + gi;
+            T* t = (T*)R + 2 * ((size_t)(gi >> 1) * C * Nz + z) + (gi & 1);  // component c: + 2 c Nz
+            T f[C][1];
+            if (l < g.NL) {
+                typename Op::In q;
+                op.template load<true>(l * Nz + z, q);
+#pragma unroll
+                for (int c = 0; c < C; ++c) f[c][0] = t[2 * c * Nz] * invV;
+                op.template apply<true>(q, l * Nz + z, f, acc);
+            } else {
+#pragma unroll
+                for (int c = 0; c < C; ++c) f[c][0] = (T)0;
+            }
+#pragma unroll
+            for (int c = 0; c < C; ++c) t[2 * c * Nz] = f[c][0];
+        }
+        __syncthreads();
+        R = fft_lines<C2, MaxR>(R, S, tw, pz, L, -1);
+        for (int i = threadIdx.x; i < nl * Hz; i += blockDim.x) {
+            const int pc = g.dHz.div(i), k = i - pc * Hz;
+            const int p = pc / C, c = pc - p * C;
+            const long long la = l0 + 2 * p;
+            C2* s = spec + (((long long)b * C + c) * g.NL + la) * Hzp + k;
+            const C2 Z = R[(size_t)pc * Nz + k];
+            const C2 Zm = R[(size_t)pc * Nz + (k == 0 ? 0 : Nz - k)];
+            if (la < g.NL) s[0] = mk<C2>((T)0.5 * (Z.x + Zm.x), (T)0.5 * (Z.y - Zm.y));
+            if (la + 1 < g.NL) s[Hzp] = mk<C2>((T)0.5 * (Z.y + Zm.y), (T)-0.5 * (Z.x - Zm.x));
+        }
+        __syncthreads();  // the next tile is loaded over this one
+    }
+    block_reduce_store<Op::NSUM>(acc, red, partials, b, gridDim.x, blockIdx.x);
+    fused_finalize(fin, ctl, partials, Op::NSUM, b);
+}
+constexpr int kZGenGrid = 148 * 8;  // CTAs per entry at most (partial sums, as kZRowsGrid)
 
 }  // namespace m3d

@@ -39,6 +39,9 @@ using namespace m3d;
 namespace m3d {
 M3D_GEN_ALL(extern, 13)
 M3D_GEN_ALL(extern, 31)
+M3D_GEN_ZMID_ALL(extern, 5)
+M3D_GEN_ZMID_ALL(extern, 13)
+M3D_GEN_ZMID_ALL(extern, 31)
 }  // namespace m3d
 
 namespace {
@@ -322,6 +325,15 @@ struct m3d_solver {
     template <typename T> bool slab_ok() const;
     template <typename T, int CC> bool plane_ok() const;
     template <typename T, int CC> bool two_pass_ok() const { return plane_ok<T, CC>() || slab_ok<T>(); }
+    template <typename T, int CC> bool mid_ok() const;
+    // sweeps whose last kernel also does the next sweep's z forward
+    template <typename T, int CC> bool fused_ok() const { return two_pass_ok<T, CC>() || mid_ok<T, CC>(); }
+    template <typename T, int CC> int launches_per_sweep(bool fused) const {
+        return !fused ? 5 : (two_pass_ok<T, CC>() ? 2 : 4);
+    }
+    template <typename T, class Op, class Fin>
+    int pass_zmid_gen(const typename Op::Args& op, Ctl* ctl, typename Cx<T>::t* sp, const Fin& fin);
+    template <typename T> int pass_zmid_inelastic(const MidJ2Args& op, Ctl* ctl, typename Cx<T>::t* sp, const FinJ2& fin);
     template <typename T, int CC, bool MIX, class Fin>
     int pass_slab(Ctl* ctl, T* x, const float* r, typename Cx<T>::t* sp, Fin fin);
     template <typename T, int CC>
@@ -711,7 +723,7 @@ void m3d_solver::pass_y(int sign, int CC, Ctl* ctl, typename Cx<T>::t* sp) {
     });
     if (!done) {
         const int tzy = TZy<T>();
-        const size_t ysmem = (size_t)Ny * sizeof(C2) + 2 * (size_t)Ny * tzy * sizeof(C2);
+        const size_t ysmem = col_tile_smem<C2>(Ny, tzy);
         const int ntzy = (g.Hzp + tzy - 1) / tzy;
         with_radix(py, [&](auto r) {
             gen_y<decltype(r)::value, T>(dim3(Nx * ntzy, CC * gridB()), plan_threads(py, tzy), ysmem, stream, g, py, tw<T>(1), sp,
@@ -789,7 +801,7 @@ int m3d_solver::pass_x(Spec op, Ctl* ctl, typename Cx<T>::t* sp) {
     });
     if (!done) {
         const int tzx = TZx<T>();
-        const size_t xsmem = (size_t)Nx * sizeof(C2) + 2 * (size_t)CC * Nx * tzx * sizeof(C2) + 16 + 32 * 32 * 8;
+        const size_t xsmem = col_tile_smem<C2>(Nx, CC * tzx) + 16 + 32 * 32 * 8;
         const int ntzx = (g.Hzp + tzx - 1) / tzx;
         nblk = Ny * ntzx;
         with_radix(px, [&](auto r) {
@@ -899,8 +911,52 @@ bool m3d_solver::plane_ok() const {
     return CC == 6 && kind == M3D_KIND_MECH && use_fast && use_slab && Nx == Ny && Ny == Nz && plane_size<T>(Nz);
 }
 
+// Other shapes: the fused z pass on the row layout (passes_zmid.cuh), four launches
+// a sweep: y forward, x turnaround, y inverse, z inverse + update + z forward.
+// Compile-time lengths up to 96 that the two-pass sweeps leave (non-cubic grids)
+// keep five passes.
+template <typename T, int CC>
+bool m3d_solver::mid_ok() const {
+    if (!use_slab) return false;
+    if (!(use_fast && fast_size(Nz))) return true;
+    return (Nz > 96 || (Nz == 96 && sizeof(T) == 8)) && zmid_rows_ok<T>(Nz, CC, g.NL);
+}
+
+template <typename T, class Op, class Fin>
+int m3d_solver::pass_zmid_gen(const typename Op::Args& op, Ctl* ctl, typename Cx<T>::t* sp, const Fin& fin) {
+    cudaError_t e = cudaSuccess;
+    constexpr int CC = std::is_same<Op, MidEM<T, 1, 3>>::value ? 3 : 6;
+    with_radix(pz, [&](auto r) {
+        e = gen_zmid<decltype(r)::value, T, CC, Op, Fin>(gridB(), stream, g, pz, tw<T>(2), sp, op, ctl, G<T>(), d_part, fin);
+    });
+    M3D_CUDA(e);
+    st.kernel_launches += 1;
+    return M3D_OK;
+}
+template <typename T>
+int m3d_solver::pass_zmid_inelastic(const MidJ2Args& op, Ctl* ctl, typename Cx<T>::t* sp, const FinJ2& fin) {
+    const bool j2 = behav == M3D_BEHAV_J2;
+    if (!(use_fast && fast_size(Nz)))
+        return j2 ? pass_zmid_gen<T, MidJ2<T, true>>(op, ctl, sp, fin) : pass_zmid_gen<T, MidJ2<T, false>>(op, ctl, sp, fin);
+    M3D_CUDA(zmid_rows_inelastic<T>(Nz, j2, gridB(), stream, g, tw<T>(2), sp, op, ctl, d_part, fin));
+    st.kernel_launches += 1;
+    return M3D_OK;
+}
+
 template <typename T, int CC, bool MIX, class Fin>
 int m3d_solver::pass_slab(Ctl* ctl, T* x, const float* r, typename Cx<T>::t* sp, Fin fin) {
+    if (!two_pass_ok<T, CC>()) {
+        if constexpr (MIX) {
+            const MidEMArgs<T> op = tab(MidEMArgs<T>{d_phase, x, r, g.V, dm(off_P), dm(off_A), nph_max()});
+            if (!(use_fast && fast_size(Nz))) return pass_zmid_gen<T, MidEM<T, 1, CC>>(op, ctl, sp, fin);
+            M3D_CUDA(zmid_rows_em<T>(Nz, CC, gridB(), stream, g, tw<T>(2), sp, op, ctl, d_part, fin));
+            st.kernel_launches += 1;
+        } else {
+            pass_zfwd<T, CC>(tab(ProMat<T, CC>{d_phase, x, g.V, dm(off_P), nph_max(), nullptr}), ctl, sp);
+            M3D_CUDA(cudaGetLastError());
+        }
+        return M3D_OK;
+    }
     if constexpr (CC == 6) {
         if (plane_ok<T, CC>()) {
             MidEMArgs<T> op = tab(MidEMArgs<T>{d_phase, x, r, g.V, dm(off_P), dm(off_A), nph_max()});
@@ -937,13 +993,17 @@ int m3d_solver::pass_slab(Ctl* ctl, T* x, const float* r, typename Cx<T>::t* sp,
     return M3D_OK;
 }
 
-// One two-pass sweep; the finalize runs in the last CTA of the slab pass.
-// Profiling slots: 2 = x turnaround, 4 = slab pass.
+// One sweep whose last kernel also does the next sweep's z forward (two passes,
+// or four with the fused z pass); the finalize runs in that kernel's last CTA.
+// Profiling slots: 1 and 3 = y passes (four-pass sweeps), 2 = x turnaround or
+// plane pass, 4 = the last kernel.
 template <typename T, int CC>
 int m3d_solver::launch_em_slab(Ctl* ctl, T* x, const float* r, typename Cx<T>::t* sp, int zero_k0, int policy,
                                const Ctl* outer) {
     prof_pass(0);
     prof_pass(1);
+    const bool four = !two_pass_ok<T, CC>();
+    if (four) pass_y<T>(-1, CC, ctl, sp);
     prof_pass(2);
     bool plane = false;
     if constexpr (CC == 6) {
@@ -955,6 +1015,7 @@ int m3d_solver::launch_em_slab(Ctl* ctl, T* x, const float* r, typename Cx<T>::t
     }
     if (!plane) pass_x<T, CC>(green<T, CC>(zero_k0), ctl, sp);
     prof_pass(3);
+    if (four) pass_y<T>(+1, CC, ctl, sp);
     prof_pass(4);
     const int rc = pass_slab<T, CC, true>(ctl, x, r, sp, FinLinear{policy, (double)g.V, outer, d_counter, loop_end});
     prof_pass(5);
@@ -982,8 +1043,8 @@ int m3d_solver::run_linear(double tol_field, double tol_eq, int criterion, int m
     C2* sp = (C2*)d_spec;
     const int chunk = kChunk;
     int before = 0;
-    const bool slab = criterion == M3D_CRIT_RESIDUAL && two_pass_ok<T, CC>();
-    st.passes_per_sweep = slab ? 2 : 5;
+    const bool slab = criterion == M3D_CRIT_RESIDUAL && fused_ok<T, CC>();
+    st.passes_per_sweep = launches_per_sweep<T, CC>(slab);
     if (slab) {
         rc = pass_slab<T, CC, false>(d_ctl, x, nullptr, sp, FinNone{});
         if (rc) return rc;
@@ -1043,8 +1104,8 @@ int m3d_solver::run_refine(double tol_field, int max_iter) {
     long long n64 = 0, n32 = 0;
     bool first = true;
     const int chunk = 8;
-    const bool slab = two_pass_ok<float, CC>();
-    st.passes_per_sweep = slab ? 2 : 5;
+    const bool slab = fused_ok<float, CC>();
+    st.passes_per_sweep = launches_per_sweep<float, CC>(slab);
     std::vector<long long> in32((size_t)B, 0);  // FP32 sweeps per entry
     for (;;) {
         ProRefine64<CC> pro = tab(ProRefine64<CC>{d_phase, x, first ? nullptr : d_delta, g.V, dm(off_P), nph_max(), nullptr});
@@ -1287,8 +1348,8 @@ int m3d_solver::run_linear_graph(double tol_field, double tol_eq, int criterion,
     k_fill_load<T><<<dim3(256, B * CC), 256, 0, stream>>>(x, d_ctl, CC, g.V);
     M3D_CUDA(cudaMemsetAsync(d_trips, 0, 8 * sizeof(int), stream));
     const bool resid = (criterion == M3D_CRIT_RESIDUAL);
-    const bool slab = resid && two_pass_ok<T, CC>();
-    st.passes_per_sweep = slab ? 2 : 5;
+    const bool slab = resid && fused_ok<T, CC>();
+    st.passes_per_sweep = launches_per_sweep<T, CC>(slab);
     if (slab) {
         rc = pass_slab<T, CC, false>(d_ctl, x, nullptr, sp, FinNone{});
         if (rc) return rc;
@@ -1357,7 +1418,7 @@ int m3d_solver::run_linear_graph(double tol_field, double tol_eq, int criterion,
     M3D_CUDA(cudaMemcpy(trips, d_trips, sizeof(trips), cudaMemcpyDeviceToHost));
     // launches per trip: the passes, of a compacted loop one more
     const int ntrips = lv.empty() ? max_iters() : trips[0];
-    st.kernel_launches += 1 + (long long)lv.size() + (long long)ntrips * ((slab ? 2 : (resid ? 5 : 9)) + (lv.empty() ? 0 : 1));
+    st.kernel_launches += 1 + (long long)lv.size() + (long long)ntrips * ((resid ? st.passes_per_sweep : 9) + (lv.empty() ? 0 : 1));
     long long sw = 0;
     int status = M3D_OK;
     for (int b = 0; b < B; ++b) {
@@ -1387,8 +1448,8 @@ int m3d_solver::run_refine_graph(double tol_field, int max_iter) {
     M3D_CUDA(cudaMemsetAsync(d_delta, 0, dbytes, stream));
     M3D_CUDA(cudaMemsetAsync(d_ctl_in, 0, (size_t)B * sizeof(Ctl), stream));
     M3D_CUDA(cudaMemsetAsync(d_trips, 0, 8 * sizeof(int), stream));
-    const bool slab = two_pass_ok<float, CC>();
-    st.passes_per_sweep = slab ? 2 : 5;
+    const bool slab = fused_ok<float, CC>();
+    st.passes_per_sweep = launches_per_sweep<float, CC>(slab);
     const size_t sbytes32 = (size_t)B * CC * g.NL * g.Hzp * sizeof(float2);
     GraphSlot& gs = gslot[2];
     const long long key = graph_key(2);
@@ -1470,7 +1531,7 @@ int m3d_solver::run_refine_graph(double tol_field, int max_iter) {
     if (rc) return rc;
     int trips[8];
     M3D_CUDA(cudaMemcpy(trips, d_trips, sizeof(trips), cudaMemcpyDeviceToHost));
-    st.kernel_launches += 1 + (long long)trips[1] * (6 + (long long)lv.size()) + (long long)trips[3] * ((slab ? 2 : 5) + (lv.empty() ? 0 : 1));
+    st.kernel_launches += 1 + (long long)trips[1] * (6 + (long long)lv.size()) + (long long)trips[3] * (st.passes_per_sweep + (lv.empty() ? 0 : 1));
     long long n64 = 0, n32 = 0;
     int status = M3D_OK;
     for (int b = 0; b < B; ++b) {
@@ -2315,7 +2376,7 @@ int m3d_solver::tune_time(int sweeps, float* ms) {
     cudaEvent_t e0, e1;
     M3D_CUDA(cudaEventCreate(&e0));
     M3D_CUDA(cudaEventCreate(&e1));
-    const bool slab = two_pass_ok<T, CC>();
+    const bool slab = fused_ok<T, CC>();
     auto sweep = [&]() {
         return slab ? launch_em_slab<T, CC>(d_ctl, x, r, sp, 0, POL_RESIDUAL, nullptr)
                     : launch_em<T, CC>(d_ctl, x, r, sp, 0, POL_RESIDUAL, nullptr);
@@ -2347,8 +2408,8 @@ int m3d_solver::autotune(int sweeps, m3d_tune* out) {
         cand.push_back(m3d_tune{1, 1, G0, Y0, X0, 0, 0, 0, 0});
         const bool f1 = use_fast, s1 = use_slab;
         use_fast = use_slab = true;
-        const bool slab_possible = fp64 ? (C == 6 ? two_pass_ok<double, 6>() : two_pass_ok<double, 3>())
-                                        : (C == 6 ? two_pass_ok<float, 6>() : two_pass_ok<float, 3>());
+        const bool slab_possible = fp64 ? (C == 6 ? fused_ok<double, 6>() : fused_ok<double, 3>())
+                                        : (C == 6 ? fused_ok<float, 6>() : fused_ok<float, 3>());
         use_fast = f1;
         use_slab = s1;
         if (slab_possible) cand.push_back(m3d_tune{1, 0, G0, Y0, X0, 0, 0, 1, 0});
@@ -2360,7 +2421,7 @@ int m3d_solver::autotune(int sweeps, m3d_tune* out) {
             if ((size_t)Nz * csz * (1 + (size_t)Gv * C) + 32 * 32 * 8 + op_smem<double, 6>() > lim) continue;
             for (int tz : {2, 4, 8, 16}) {
                 if (2 * (size_t)C * Nx * tz * csz + (size_t)Nx * csz > lim || 2 * (size_t)Ny * tz * csz > lim) continue;
-                cand.push_back(m3d_tune{0, 0, Gv, tz, tz, 0, 0, 0, 0});
+                cand.push_back(m3d_tune{0, 0, Gv, tz, tz, 0, 0, 1, 0});
             }
         }
         auto same = [](const LinePlan& a, const LinePlan& b) {
@@ -2376,7 +2437,7 @@ int m3d_solver::autotune(int sweeps, m3d_tune* out) {
             for (int o2 = 0; o2 < o && !dup; ++o2)
                 if (make_plan(Nx, rx, o2) && make_plan(Ny, ry, o2) && make_plan(Nz, rz, o2))
                     dup = same(qx, rx) && same(qy, ry) && same(qz, rz);
-            if (!dup) cand.push_back(m3d_tune{0, 0, G0, Y0, X0, 0, 0, 0, o});
+            if (!dup) cand.push_back(m3d_tune{0, 0, G0, Y0, X0, 0, 0, 1, o});
         }
     }
     const bool f0 = use_fast, t0 = use_tma_y, sl0 = use_slab;

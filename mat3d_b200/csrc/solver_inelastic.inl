@@ -180,9 +180,9 @@ int m3d_solver::run_inelastic(double tol_field, double tol_eq, int nInc, int cri
     // stress increment (J2 keeps the previous step's stress)
     if (sizeof(T) == 4 && criterion == M3D_CRIT_RESIDUAL && sig_old) pro.sig_old = sig_old;
     SpecBasic<T> spec{green<T, 6>(0), SpecEqVar<T, 6>{g}};
-    // fused z pass (z inverse, update, next z forward) where Nz has one; the
-    // stress then stays in registers and is written at the end of an increment
-    const bool mid = use_fast && use_slab && zmid_rows_ok<T>(Nz, g.NL);
+    // fused z pass (z inverse, update, next z forward): every length but the
+    // compile-time ones whose tiles the lines do not fill; the stress then stays in registers and is written at the end of an increment
+    const bool mid = use_slab && (!(use_fast && fast_size(Nz)) || zmid_rows_ok<T>(Nz, 6, g.NL));
     const MidJ2Args margs{d_phase, eps, eps_old, sig_old, ep, dmg, V, in.d_ph, nph, pro.sig_old ? 1 : 0, in.d_nrfail};
     // the convergence sums of the stress spectrum are the reference rule's alone
     const bool check = criterion == M3D_CRIT_REFERENCE;
@@ -229,9 +229,8 @@ int m3d_solver::run_inelastic(double tol_field, double tol_eq, int nInc, int cri
                 prof_pass(4);
                 const FinJ2 fin{POLJ2_SWEEP, (double)V, in.d_S0, d_counter};
                 if (mid) {
-                    M3D_CUDA(zmid_rows_inelastic<T>(Nz, behav == M3D_BEHAV_J2, B, stream, g, tw<T>(2), sp, margs, d_ctl,
-                                                    d_part, fin));
-                    st.kernel_launches += 1;
+                    const int zrc = pass_zmid_inelastic<T>(margs, d_ctl, sp, fin);
+                    if (zrc) return zrc;
                 } else {
                     pass_zinv<T, 6>(epi, d_ctl, sp, fin);
                 }

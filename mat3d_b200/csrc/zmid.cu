@@ -1,7 +1,4 @@
 // zmid.cu -- the fused z pass on the row layout: kernels and launches.
-#include <algorithm>
-
-#include "generic_launch.cuh"  // allow_smem
 #include "zmid_launch.cuh"
 
 namespace m3d {
@@ -30,14 +27,48 @@ cudaError_t go(int entries, cudaStream_t st, const GridDims& g, const typename C
 }
 }  // namespace
 
+// The EM kernels are for the shapes that the two-pass sweeps (passes_plane.cuh,
+// passes_slab.cuh) do not cover; at 96 points and below five passes remain only
+// for non-cubic grids.
+template <typename T, int C, class F> void with_em_n(int n, F&& f) {
+    switch (n) {
+        case 96: if constexpr (sizeof(T) == 8) f(IntC<96>{}); break;
+        case 128: if constexpr (sizeof(T) == 8 || C == 6) f(IntC<128>{}); break;
+        case 256: f(IntC<256>{}); break;
+        default: break;
+    }
+}
 template <typename T>
-bool zmid_rows_ok(int N, long long NL) {
+bool zmid_rows_ok(int N, int C, long long NL) {
     bool ok = false;
-    with_n(N, [&](auto nc) { ok = NL % ZRowsGeom<T, decltype(nc)::value, 6>::G == 0; });
+    if (C == 6) with_n(N, [&](auto nc) { ok = NL % ZRowsGeom<T, decltype(nc)::value, 6>::G == 0; });
+    else with_em_n<T, 3>(N, [&](auto nc) { ok = NL % ZRowsGeom<T, decltype(nc)::value, 3>::G == 0; });
     return ok;
 }
-template bool zmid_rows_ok<float>(int, long long);
-template bool zmid_rows_ok<double>(int, long long);
+template bool zmid_rows_ok<float>(int, int, long long);
+template bool zmid_rows_ok<double>(int, int, long long);
+
+template <typename T>
+cudaError_t zmid_rows_em(int N, int C, int entries, cudaStream_t st, const GridDims& g, const typename Cx<T>::t* tw,
+                         typename Cx<T>::t* sp, const MidEMArgs<T>& op, Ctl* ctl, double* part, const FinLinear& fin) {
+    cudaError_t e = cudaErrorInvalidValue;
+    constexpr int W = sizeof(T) == 4 ? 2 : 1;
+    if (C == 6)
+        with_em_n<T, 6>(N, [&](auto nc) {
+            e = go<T, decltype(nc)::value, 6, MidEM<T, W, 6>, FinLinear>(entries, st, g, tw, sp, op, ctl, part, fin);
+        });
+    else
+        with_em_n<T, 3>(N, [&](auto nc) {
+            e = go<T, decltype(nc)::value, 3, MidEM<T, W, 3>, FinLinear>(entries, st, g, tw, sp, op, ctl, part, fin);
+        });
+    return e;
+}
+template cudaError_t zmid_rows_em<float>(int, int, int, cudaStream_t, const GridDims&, const float2*, float2*,
+                                         const MidEMArgs<float>&, Ctl*, double*, const FinLinear&);
+template cudaError_t zmid_rows_em<double>(int, int, int, cudaStream_t, const GridDims&, const double2*, double2*,
+                                          const MidEMArgs<double>&, Ctl*, double*, const FinLinear&);
+
+M3D_GEN_ZMID_ALL(, 5)
 
 template <typename T>
 cudaError_t zmid_rows_inelastic(int N, bool j2, int entries, cudaStream_t st, const GridDims& g,
