@@ -84,12 +84,12 @@ inline bool make_plan(int n, LinePlan& p, int order = 0) {
 }
 
 // Threads of a CTA that transforms `lines` lines of plan p together: one per
-// butterfly of its widest stage, 64 to 256.
-inline int plan_threads(const LinePlan& p, int lines) {
+// butterfly of its widest stage, 64 to `most`.
+inline int plan_threads(const LinePlan& p, int lines, int most = 256) {
     int r = 1;
     for (int s = 0; s < p.nstages; ++s) r = std::max(r, p.radix[s]);
     const int b = lines * (p.n / r);
-    return std::max(64, std::min(256, (b + 31) / 32 * 32));
+    return std::max(64, std::min(most, (b + 31) / 32 * 32));
 }
 
 // tw[m] = exp(-2 pi i m / n), evaluated in long double

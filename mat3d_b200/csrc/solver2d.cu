@@ -5,11 +5,13 @@
 // for a fixed number of iterations, and the 3-load-case homogenization.
 //
 // Layout: complex FP64 fields component-major, f[c*xy + v], v = y + Ny*x
-// (the reference's voxel order).  One iteration = 4 launches: the pointwise
-// constitutive step, forward FFTs of the rows (y), the column turnaround (x
-// forward FFT, Green operator, x inverse FFT) and inverse FFTs of the rows
-// with the 1/xy scaling.  Transforms are the generic shared-memory Stockham
-// line FFTs (any length with prime factors up to 32).
+// (the reference's voxel order).  One iteration = 2 launches: the column
+// turnaround (x forward FFT, Green operator, x inverse FFT), and the inverse
+// FFTs of the rows with the 1/xy scaling, the pointwise constitutive step and
+// the next iteration's forward FFTs of the rows; 4 launches, the pointwise step
+// and the two row transforms apart, for rows too long to hold three of them twice
+// (above 2011 points).  Transforms are the generic shared-memory Stockham line FFTs
+// (any length with prime factors up to 32).
 //
 // The Green operator follows setGF/multiplyGF (:49-137) including their
 // conventions: frequencies x <= (Nx-1)/2 positive else -(Ny - x) (x wraps with
@@ -146,66 +148,162 @@ __global__ void __launch_bounds__(256) k2d_rows(double2* __restrict__ buf, doubl
     cp_wait_all();
 }
 
+// -Gamma0 : tau^ of mode (x, y), k = 0 -> E * xy (setGF :49-103, multiplyGF :105-138)
+__device__ __forceinline__ void green2d(const double2 (&t)[3], double2 (&u)[3], int x, int y, int Nx, int Ny,
+                                        const Consts2D& k, long long xy) {
+    if (x == 0 && y == 0) {
+#pragma unroll
+        for (int c = 0; c < 3; ++c) u[c] = make_double2(k.E[c].x * (double)xy, k.E[c].y * (double)xy);
+    } else {
+        const double z[2] = {(double)(x <= (Nx - 1) / 2 ? x : -(Ny - x)), (double)(y <= (Ny - 1) / 2 ? y : -(Ny - y))};
+        const double n2 = z[0] * z[0] + z[1] * z[1];
+        const int q[6][4] = {{0, 0, 0, 0}, {0, 0, 1, 1}, {0, 0, 0, 1}, {1, 1, 1, 1}, {1, 1, 0, 1}, {0, 1, 0, 1}};
+        double gf[6];
+#pragma unroll
+        for (int s = 0; s < 6; ++s) {
+            const int a = q[s][0], b = q[s][1], c = q[s][2], h = q[s][3];
+            gf[s] = (k.d1 / n2) * ((c == a ? 1.0 : 0.0) * z[h] * z[b] + (h == a ? 1.0 : 0.0) * z[c] * z[b] +
+                                   (c == b ? 1.0 : 0.0) * z[h] * z[a] + (h == b ? 1.0 : 0.0) * z[c] * z[a]) -
+                    (k.d2 * z[a] * z[b] * z[c] * z[h]) / (n2 * n2);
+        }
+        const int w[3][3] = {{0, 1, 2}, {1, 3, 4}, {2, 4, 5}};
+#pragma unroll
+        for (int j = 0; j < 3; ++j) {
+            u[j].x = -(gf[w[j][0]] * t[0].x + gf[w[j][1]] * t[1].x + gf[w[j][2]] * t[2].x * 2);
+            u[j].y = -(gf[w[j][0]] * t[0].y + gf[w[j][1]] * t[1].y + gf[w[j][2]] * t[2].y * 2);
+        }
+    }
+}
+
 // Column turnaround: TZ consecutive columns y of all Nx rows and 3 components;
 // forward FFT along x, -Gamma0 : tau^ per mode (k = 0 -> E * xy), inverse FFT.
+// Point x of line 3 tz + c lies at 3 TZ x + 3 tz + c and consecutive threads take
+// the lines of one point, then the next point's: a first stage of radix 8 or 16,
+// whose outputs lie that far apart, then has at most 2-way bank conflicts where
+// threads along one line had 8-way ones.  Bound by the latency of one CTA's stages
+// (200 KB of shared memory at 1024: one CTA per SM).  At 1024^2 165 us before (one
+// column and 256 threads a CTA), 100 us now; 50 MB in and out are in L2.
+// A thread per butterfly, up to 512; the radices above 13 want 255 registers.
+constexpr int cols_most(int max_r) { return max_r > 13 ? 256 : 512; }
 template <int MaxR>
-__global__ void __launch_bounds__(256) k2d_cols(double2* __restrict__ buf, const double2* __restrict__ twx, const __grid_constant__ LinePlan px, int Ny, FastDiv dTZ,
+__global__ void __launch_bounds__(cols_most(MaxR), 1) k2d_cols(double2* __restrict__ buf, const double2* __restrict__ twx, const __grid_constant__ LinePlan px, int Ny, FastDiv dTZ,
                          Consts2D k, long long xy) {
     extern __shared__ __align__(16) char smem_raw[];
     const int Nx = px.n, TZ = dTZ.d;
     double2* tw = (double2*)smem_raw;
-    double2* A = tw + Nx;  // [c][x][tz]
+    double2* A = tw + Nx;  // [x][tz][c]
     double2* B = A + (size_t)3 * Nx * TZ;
     const int y0 = blockIdx.x * TZ;
+    for (int c = 0; c < 3; ++c)
+        for (int i = threadIdx.x; i < Nx * TZ; i += blockDim.x) {
+            const int x = dTZ.div(i), y = y0 + i - x * TZ;
+            cp16(A + 3 * i + c, buf + c * xy + (long long)x * Ny + (y < Ny ? y : y0), y < Ny);
+        }
+    cp_commit();
     for (int i = threadIdx.x; i < Nx; i += blockDim.x) tw[i] = twx[i];
-    for (int i = threadIdx.x; i < 3 * Nx * TZ; i += blockDim.x) {
-        const int cx = dTZ.div(i), tz = i - cx * TZ, c = px.dn.div(cx), x = cx - c * Nx;
-        const int y = y0 + tz;
-        A[i] = y < Ny ? buf[c * xy + (long long)x * Ny + y] : make_double2(0, 0);
-    }
+    cp_wait_all();
     __syncthreads();
-    LineLayout L{3 * TZ, TZ, 1, Nx * TZ, TZ, false};
+    const LineLayout L{3 * TZ, 3 * TZ, 1, 0, 3 * TZ, true};
     double2* r = fft_lines<double2, MaxR>(A, B, tw, px, L, -1);
     double2* o = (r == A) ? B : A;
-    // Green operator (setGF :49-103, multiplyGF :105-138)
     for (int i = threadIdx.x; i < Nx * TZ; i += blockDim.x) {
         const int x = dTZ.div(i), tz = i - x * TZ, y = y0 + tz;
         double2 t[3];
 #pragma unroll
-        for (int c = 0; c < 3; ++c) t[c] = r[(c * Nx + x) * TZ + tz];
+        for (int c = 0; c < 3; ++c) t[c] = r[3 * i + c];
         double2 u[3];
-        if (x == 0 && y == 0) {
+        green2d(t, u, x, y, Nx, Ny, k, xy);
 #pragma unroll
-            for (int c = 0; c < 3; ++c) u[c] = make_double2(k.E[c].x * (double)xy, k.E[c].y * (double)xy);
-        } else {
-            const double z[2] = {(double)(x <= (Nx - 1) / 2 ? x : -(Ny - x)), (double)(y <= (Ny - 1) / 2 ? y : -(Ny - y))};
-            const double n2 = z[0] * z[0] + z[1] * z[1];
-            const int q[6][4] = {{0, 0, 0, 0}, {0, 0, 1, 1}, {0, 0, 0, 1}, {1, 1, 1, 1}, {1, 1, 0, 1}, {0, 1, 0, 1}};
-            double gf[6];
-#pragma unroll
-            for (int s = 0; s < 6; ++s) {
-                const int a = q[s][0], b = q[s][1], c = q[s][2], h = q[s][3];
-                gf[s] = (k.d1 / n2) * ((c == a ? 1.0 : 0.0) * z[h] * z[b] + (h == a ? 1.0 : 0.0) * z[c] * z[b] +
-                                       (c == b ? 1.0 : 0.0) * z[h] * z[a] + (h == b ? 1.0 : 0.0) * z[c] * z[a]) -
-                        (k.d2 * z[a] * z[b] * z[c] * z[h]) / (n2 * n2);
-            }
-            const int w[3][3] = {{0, 1, 2}, {1, 3, 4}, {2, 4, 5}};
-#pragma unroll
-            for (int j = 0; j < 3; ++j) {
-                u[j].x = -(gf[w[j][0]] * t[0].x + gf[w[j][1]] * t[1].x + gf[w[j][2]] * t[2].x * 2);
-                u[j].y = -(gf[w[j][0]] * t[0].y + gf[w[j][1]] * t[1].y + gf[w[j][2]] * t[2].y * 2);
-            }
-        }
-#pragma unroll
-        for (int c = 0; c < 3; ++c) o[(c * Nx + x) * TZ + tz] = u[c];
+        for (int c = 0; c < 3; ++c) o[3 * i + c] = u[c];
     }
     __syncthreads();
     double2* s = fft_lines<double2, MaxR>(o, r, tw, px, L, +1);
-    for (int i = threadIdx.x; i < 3 * Nx * TZ; i += blockDim.x) {
-        const int cx = dTZ.div(i), tz = i - cx * TZ, c = px.dn.div(cx), x = cx - c * Nx;
-        const int y = y0 + tz;
-        if (y < Ny) buf[c * xy + (long long)x * Ny + y] = s[i];
+    for (int c = 0; c < 3; ++c)
+        for (int i = threadIdx.x; i < Nx * TZ; i += blockDim.x) {
+            const int x = dTZ.div(i), y = y0 + i - x * TZ;
+            if (y < Ny) buf[c * xy + (long long)x * Ny + y] = s[3 * i + c];
+        }
+}
+
+// ---------------------------------------------------------------------------
+// The rows of one iteration's end and the next one's start in one kernel: inverse
+// rows, sigma = C(x) eps, tau, forward rows, so that the strain and tau do not
+// pass through memory and sigma is stored once per run.
+// FIRST: from the strain field; LAST: to the strain field; else both halves.
+// sig: where sigma goes (null: not stored).  A CTA has g rows of three
+// components; point y of line 3 r + c lies at 3 g y + 3 r + c, so that consecutive
+// threads take the lines of one point, then the next point's: at most 3-way bank
+// conflicts in a first stage, whose outputs lie a radix apart, where threads along a
+// row had 8-way ones (116 us at 1024^2), and none in the copies (3 g is odd).
+// Bound by the latency of a CTA's stages, 98 KB and two CTAs per SM at 1024.  At
+// 1024^2 98 us; the pointwise step and the two row transforms apart took 24 + 55 + 61.
+// ---------------------------------------------------------------------------
+enum RowsMode { ROWS_FIRST = 0, ROWS_MID = 1, ROWS_LAST = 2 };
+template <int MaxR>
+__global__ void __launch_bounds__(256) k2d_mid(double2* __restrict__ buf, double2* __restrict__ eps,
+                                                      double2* __restrict__ sig, const uint8_t* __restrict__ phase,
+                                                      const double2* __restrict__ twy, const __grid_constant__ LinePlan py,
+                                                      int g, int Nx, const __grid_constant__ Consts2D k, long long xy,
+                                               RowsMode mode) {
+    extern __shared__ __align__(16) char smem_raw[];
+    const int Ny = py.n;
+    double2* A = (double2*)smem_raw;
+    double2* B = A + 3 * g * Ny;
+    double2* tw = B + 3 * g * Ny;
+    const int x0 = blockIdx.x * g, rows = min(g, Nx - x0), nv = rows * Ny;
+    const long long v0 = (long long)x0 * Ny;  // the rows of a component are one run
+    const double2* src = mode == ROWS_FIRST ? eps : buf;
+    const int es = 3 * g;
+    for (int c = 0; c < 3; ++c)
+        for (int i = threadIdx.x; i < g * Ny; i += blockDim.x) {
+            const int r = py.dn.div(i);
+            cp16(A + (i - r * Ny) * es + 3 * r + c, src + c * xy + v0 + (i < nv ? i : 0), i < nv);
+        }
+    cp_commit();
+    for (int i = threadIdx.x; i < Ny; i += blockDim.x) tw[i] = twy[i];
+    const LineLayout L{es, es, 1, 0, es, true};
+    cp_wait_all();
+    __syncthreads();
+    double2* R = A;
+    if (mode != ROWS_FIRST) R = fft_lines<double2, MaxR>(A, B, tw, py, L, +1);
+    const double dxy = (double)xy;
+    for (int i = threadIdx.x; i < nv; i += blockDim.x) {
+        const int row = py.dn.div(i);
+        double2* p = R + (i - row * Ny) * es + 3 * row;
+        double2 e[3];
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+            e[c] = p[c];
+            if (mode != ROWS_FIRST) e[c] = make_double2(e[c].x / dxy, e[c].y / dxy);  // FFTBCKWRD_epsilon :140-145
+        }
+        if (mode == ROWS_LAST) {
+#pragma unroll
+            for (int c = 0; c < 3; ++c) eps[c * xy + v0 + i] = e[c];
+            continue;
+        }
+        const double* M = phase[v0 + i] ? k.Cm : k.Ci;
+#pragma unroll
+        for (int r = 0; r < 3; ++r) {
+            double sr = 0, si = 0, tr = 0, ti = 0;
+#pragma unroll
+            for (int j = 0; j < 3; ++j) {
+                sr += M[r * 3 + j] * e[j].x;
+                si += M[r * 3 + j] * e[j].y;
+                tr += k.C0[r * 3 + j] * e[j].x;
+                ti += k.C0[r * 3 + j] * e[j].y;
+            }
+            if (sig) sig[r * xy + v0 + i] = make_double2(sr, si);
+            p[r] = make_double2(sr - tr, si - ti);
+        }
     }
+    if (mode == ROWS_LAST) return;
+    __syncthreads();
+    R = fft_lines<double2, MaxR>(R, R == A ? B : A, tw, py, L, -1);
+    for (int c = 0; c < 3; ++c)
+        for (int i = threadIdx.x; i < nv; i += blockDim.x) {
+            const int r = py.dn.div(i);
+            buf[c * xy + v0 + i] = R[(i - r * Ny) * es + 3 * r + c];
+        }
 }
 
 // per-block sums of the real parts of eps and sigma (6 values)
@@ -218,16 +316,8 @@ __global__ void k2d_means(const double2* __restrict__ eps, const double2* __rest
             a[c] += eps[c * xy + v].x;
             a[3 + c] += sig[c * xy + v].x;
         }
-    __shared__ double red[6][256];
-#pragma unroll
-    for (int s = 0; s < 6; ++s) red[s][threadIdx.x] = a[s];
-    __syncthreads();
-    if (threadIdx.x == 0)
-        for (int s = 0; s < 6; ++s) {
-            double t = 0;
-            for (int i = 0; i < (int)blockDim.x; ++i) t += red[s][i];
-            part[s * gridDim.x + blockIdx.x] = t;
-        }
+    __shared__ double red[6 * 32];
+    block_reduce_store<6>(a, red, part, 0, gridDim.x, blockIdx.x);
 }
 
 // AoS export: out[(v*3 + c)] = f[c*xy + v]
@@ -289,6 +379,42 @@ struct m3d_solver2d {
     }
     int rows_nbuf = 3;  // shared buffers of the row passes (3: the next tile prefetched)
     int rows_grid = 1;  // persistent CTAs of the row passes
+    int g_mid = 0, nt_mid = 256, nt_cols = 256;  // fused rows per CTA (0: a row too long for them), threads
+    size_t mid_smem() const { return (size_t)(6 * g_mid + 1) * Ny * 16; }
+    // Fused rows: up to 48 KB a buffer (two CTAs per SM), an odd number, and two CTAs
+    // for every SM before a CTA takes a third row.  They are the faster at every size:
+    // 25 iterations took 3.58 -> 1.73 ms at 64^2, 3.42 -> 3.01 at 171^2, 6.8 -> 4.5 at
+    // 512^2, 23.9 -> 15.4 at 1024^2 (with the columns' tiles).
+    void pick_mid() {
+        g_mid = std::max(1, std::min(std::min(16, (int)(48 * 1024 / (48 * (size_t)Ny))), Nx / 296));
+        g_mid -= g_mid % 2 == 0;
+        if (mid_smem() > 220 * 1024) g_mid = 0;
+        nt_mid = plan_threads(py, 3 * std::max(1, g_mid));
+    }
+    int rows_mid(RowsMode mode, double2* s) {
+        with_radix(py, [&](auto r) {
+            k2d_mid<decltype(r)::value><<<(Nx + g_mid - 1) / g_mid, nt_mid, mid_smem(), stream>>>(buf, eps, s, phase, twy, py, g_mid,
+                                                                                                 Nx, k, xy, mode);
+        });
+        launches += 1;
+        M2_CUDA(cudaGetLastError());
+        return M3D_OK;
+    }
+    void cols() {
+        with_radix(px, [&](auto r) {
+            k2d_cols<decltype(r)::value><<<(Ny + TZ - 1) / TZ, nt_cols, cols_smem(), stream>>>(buf, twx, px, Ny, fast_div(TZ), k, xy);
+        });
+        launches += 1;
+    }
+    int run_mid(int iterations) {
+        int rc = rows_mid(ROWS_FIRST, iterations == 1 ? sig : nullptr);
+        for (int i = 1; i <= iterations && !rc; ++i) {
+            cols();
+            // sigma of a run is that of the strain its last iteration starts from
+            rc = i == iterations ? rows_mid(ROWS_LAST, nullptr) : rows_mid(ROWS_MID, i + 1 == iterations ? sig : nullptr);
+        }
+        return rc;
+    }
     size_t rows_smem() const { return (size_t)Ny * 16 + (size_t)rows_nbuf * G * Ny * 16; }
     size_t cols_smem() const { return (size_t)Nx * 16 + 2 * (size_t)3 * Nx * TZ * 16; }
     int iterate() {
@@ -298,13 +424,11 @@ struct m3d_solver2d {
         with_radix(py, [&](auto r) {
             k2d_rows<decltype(r)::value><<<rows_grid, 256, rows_smem(), stream>>>(buf, nullptr, twy, py, G, nlines, -1, xy, rows_nbuf);
         });
-        with_radix(px, [&](auto r) {
-            k2d_cols<decltype(r)::value><<<(Ny + TZ - 1) / TZ, 256, cols_smem(), stream>>>(buf, twx, px, Ny, fast_div(TZ), k, xy);
-        });
+        cols();
         with_radix(py, [&](auto r) {
             k2d_rows<decltype(r)::value><<<rows_grid, 256, rows_smem(), stream>>>(buf, eps, twy, py, G, nlines, +1, xy, rows_nbuf);
         });
-        launches += 4;
+        launches += 3;
         M2_CUDA(cudaGetLastError());
         return M3D_OK;
     }
@@ -330,10 +454,18 @@ int m3d2d_create(int Nx, int Ny, m3d_solver2d** out) {
     h->G = std::max(1, std::min(16, (int)(48 * 1024 / (32 * (size_t)Ny))));
     if ((size_t)Ny * 16 + 3 * (size_t)h->G * Ny * 16 > 220 * 1024) h->rows_nbuf = 2;
     h->TZ = std::max(1, std::min(16, (int)(96 * 1024 / (96 * (size_t)Nx))));
-    if (h->rows_smem() > 220 * 1024 || h->cols_smem() > 220 * 1024) {
+    const bool fits = h->rows_smem() <= 220 * 1024 && h->cols_smem() <= 220 * 1024;
+    // two columns make whole 32-byte sectors
+    if (h->TZ == 1 && fits) {
+        h->TZ = 2;
+        if (h->cols_smem() > 220 * 1024) h->TZ = 1;
+    }
+    with_radix(h->px, [&](auto r) { h->nt_cols = plan_threads(h->px, 3 * h->TZ, cols_most(decltype(r)::value)); });
+    if (!fits) {
         delete h;
         return fail2d(M3D_ERR_UNSUPPORTED, "grid too large for the shared-memory line FFTs");
     }
+    h->pick_mid();
     const size_t f = (size_t)3 * h->xy * sizeof(double2);
     if (cudaStreamCreateWithFlags(&h->stream, cudaStreamNonBlocking) != cudaSuccess ||
         cudaMalloc(&h->eps, f) != cudaSuccess || cudaMalloc(&h->sig, f) != cudaSuccess ||
@@ -352,9 +484,13 @@ int m3d2d_create(int Nx, int Ny, m3d_solver2d** out) {
     cudaMemset(h->sig, 0, f);
     // one limit per kernel for every handle (a per-handle value would lower it
     // under a larger handle made earlier): the device maximum
-    with_radix(h->py, [&](auto r) { allow_smem(k2d_rows<decltype(r)::value>); });
     with_radix(h->px, [&](auto r) { allow_smem(k2d_cols<decltype(r)::value>); });
-    {
+    with_radix(h->py, [&](auto r) {
+        // (only of the kernel the handle will run: the first such call loads it)
+        if (h->g_mid) allow_smem(k2d_mid<decltype(r)::value>);
+        else allow_smem(k2d_rows<decltype(r)::value>);
+    });
+    if (!h->g_mid) {
         int per_sm = 0, sms = 0, dev = 0;
         cudaGetDevice(&dev);
         with_radix(h->py, [&](auto r) {
@@ -419,9 +555,14 @@ int m3d2d_run(m3d_solver2d* h, int iterations) {
     if (!h) return fail2d(M3D_ERR_ARG, "NULL handle");
     if (!h->material_set || !h->load_set) return fail2d(M3D_ERR_STATE, "material and load must be set first");
     if (iterations < 1 || iterations > 100000) return fail2d(M3D_ERR_ARG, "iterations must be in [1, 100000]");
-    for (int i = 0; i < iterations; ++i) {
-        const int rc = h->iterate();
+    if (h->g_mid) {
+        const int rc = h->run_mid(iterations);
         if (rc) return rc;
+    } else {
+        for (int i = 0; i < iterations; ++i) {
+            const int rc = h->iterate();
+            if (rc) return rc;
+        }
     }
     M2_CUDA(cudaStreamSynchronize(h->stream));
     return M3D_OK;
