@@ -447,7 +447,16 @@ __global__ void __launch_bounds__(32 * kXRegWarps) k_xturn_reg(GridDims g, const
 // it: D(0) = 0 and the missing constant is added to every x.  Arithmetic is
 // the same to rounding (FP32 and FP64); the wave vectors follow SpecGreen's sign and
 // wrap rules exactly.
+// The three kernels below give equal bits, so that a batch may take any: what the
+// compiler could fuse in one and not in another is written out.
 // ---------------------------------------------------------------------------
+__device__ __forceinline__ float r1_fma(float a, float b, float c) { return __fmaf_rn(a, b, c); }
+__device__ __forceinline__ double r1_fma(double a, double b, double c) { return __fma_rn(a, b, c); }
+__device__ __forceinline__ float r1_mul(float a, float b) { return __fmul_rn(a, b); }
+__device__ __forceinline__ double r1_mul(double a, double b) { return __dmul_rn(a, b); }
+template <typename T, class C2> __device__ __forceinline__ C2 r1_add(C2 a, T f, C2 v) { return mk<C2>(r1_fma(f, v.x, a.x), r1_fma(f, v.y, a.y)); }
+template <typename T, class C2> __device__ __forceinline__ C2 r1_scale(T f, C2 v) { return mk<C2>(r1_mul(f, v.x), r1_mul(f, v.y)); }
+template <typename T> __device__ __forceinline__ T r1_norm2(T a, T b, T c) { return r1_fma(c, c, r1_fma(b, b, r1_mul(a, a))); }
 // CTAs per SM the rank-one x turnaround is compiled for (bounds its registers;
 // an FP64 lane holds twice the registers per point)
 template <typename T, int N> struct XR1MinB {
@@ -514,17 +523,17 @@ __global__ void __launch_bounds__(32 * kXRegWarps, XR1MinB<T, N>::value) k_xturn
 #pragma unroll
         for (int r = 0; r < E; ++r) {
             const T fc = c == 2 ? fx[r] : fcol;
-            d[r] = mk<C2>(d[r].x + fc * v[r].x, d[r].y + fc * v[r].y);
+            d[r] = r1_add(d[r], fc, v[r]);
         }
     }
     // D = coef d per mode; the x-frequency weighted copy for the x component
 #pragma unroll
     for (int r = 0; r < E; ++r) {
         const int mode = spec_mode<E, TL>(t, r);
-        const T n2 = fz * fz + fy * fy + fx[r] * fx[r];
+        const T n2 = r1_norm2(fz, fy, fx[r]);
         const T coef = (origin && mode == 0) ? (T)0 : (grad ? -op.p1 : (T)1) / n2;
-        d[r] = mk<C2>(coef * d[r].x, coef * d[r].y);
-        v[r] = mk<C2>(fx[r] * d[r].x, fx[r] * d[r].y);
+        d[r] = r1_scale(coef, d[r]);
+        v[r] = r1_scale(fx[r], d[r]);
     }
     // the k = 0 mode's value (the load, or 0 in a correction solve) minus what
     // the rank-one terms give there (0, and -p1 N mean for the flux form)
@@ -533,7 +542,7 @@ __global__ void __launch_bounds__(32 * kXRegWarps, XR1MinB<T, N>::value) k_xturn
 #pragma unroll
         for (int c = 0; c < C; ++c) {
             const T kc = op.zero_k0 ? (T)0 : (T)ctl[b].kzero[c];
-            add[c] = grad ? mk<C2>(kc, 0) : mk<C2>(kc + op.p1 * k0[c].x, op.p1 * k0[c].y);
+            add[c] = grad ? mk<C2>(kc, 0) : r1_add(mk<C2>(kc, 0), op.p1, k0[c]);
         }
     }
     const T sc = grad ? (T)1 : op.p1;  // scale of the rank-one terms
@@ -542,12 +551,9 @@ __global__ void __launch_bounds__(32 * kXRegWarps, XR1MinB<T, N>::value) k_xturn
 #pragma unroll
         for (int j = 0; j < E; ++j) {
             C2* p = base + c * cstride + (long long)(t + TL * j) * xstride;
-            C2 o = mk<C2>(sc * f * u[j].x, sc * f * u[j].y);
-            if (!grad) {
-                const C2 in = *p;
-                o = mk<C2>(o.x - op.p1 * (T)N * in.x, o.y - op.p1 * (T)N * in.y);
-            }
-            *p = mk<C2>(o.x + add[c].x, o.y + add[c].y);
+            C2 o = r1_scale(sc * f, u[j]);
+            if (!grad) o = r1_add(o, -(op.p1 * (T)N), *p);
+            *p = r1_add(o, (T)1, add[c]);
         }
     };
     line_inv<C2, E, TL>(d, t, xl, tw, sw);  // IFFT(D), natural order
@@ -557,6 +563,94 @@ __global__ void __launch_bounds__(32 * kXRegWarps, XR1MinB<T, N>::value) k_xturn
     }
     line_inv<C2, E, TL>(v, t, xl, tw, sw);  // IFFT(xi_x D)
     if (ok) emit(2, v, (T)1);
+}
+
+// ---------------------------------------------------------------------------
+// The rank-one x turnaround of few column groups: a CTA has one, a warp each
+// component.  The warps transform their components side by side, exchange the
+// modes through shared memory (a lane of each warp holds the same modes) and each
+// forms D for the inverse that its component needs: IFFT(xi_x D) the x component's,
+// IFFT(D) the other two, a transform more than k_xturn_r1 but three chains of one
+// transform after another instead of one of five.  Bound by that latency: 32^3 FP64
+// (24 CTAs -> 96) 8.9 -> 6.1 us a launch.  The arithmetic is k_xturn_r1's, operation for
+// operation, so the two give equal bits and a batch may take either.
+// ---------------------------------------------------------------------------
+template <typename T, int N>
+constexpr size_t xturn_r1cp_smem() {
+    constexpr int E = LineSplit<T, N>::E, CPW = 32 / LineSplit<T, N>::Tl;
+    return (size_t)(N + 3 * E * 32 + 3 * CPW * RowLen<T, N, true>::value) * sizeof(typename Cx<T>::t);
+}
+template <typename T, int N>
+__global__ void __launch_bounds__(96, 4) k_xturn_r1cp(GridDims g, const typename Cx<T>::t* __restrict__ twx,
+                                                      typename Cx<T>::t* __restrict__ spec, SpecGreenT<T> op,
+                                                      const Ctl* __restrict__ ctl) {
+    typedef typename Cx<T>::t C2;
+    constexpr int C = 3;
+    constexpr int E = LineSplit<T, N>::E, TL = LineSplit<T, N>::Tl, CPW = 32 / TL;
+    constexpr int RL = RowLen<T, N, true>::value;
+    const int b = entry_of(g, blockIdx.y);
+    if (b < 0 || ctl[b].done) return;
+    op.prepare(ctl, b);
+    extern __shared__ __align__(16) char smem_raw[];
+    C2* tw = (C2*)smem_raw;
+    C2* modes = tw + N;  // [c][r][lane]
+    C2* xch = modes + C * E * 32;
+    const int c = threadIdx.x >> 5, lane = threadIdx.x & 31;  // component `c`
+    const int col = lane % CPW, t = lane / CPW;
+    const int ngrp = (g.Hzp + CPW - 1) / CPW;
+    const int y = blockIdx.x / ngrp;
+    const int kz = (blockIdx.x - y * ngrp) * CPW + col;
+    const bool ok = kz < g.Hzp;
+    const long long xstride = (long long)g.Ny * g.Hzp;
+    C2* base = spec + (((long long)b * C + c) * g.NL + y) * g.Hzp + (ok ? kz : 0);
+    C2* xl = xch + (c * CPW + col) * RL;
+    const int sw = RowLen<T, N, true>::sw ? (col & 1) : 0;
+    C2 v[E];
+#pragma unroll
+    for (int j = 0; j < E; ++j) v[j] = ok ? base[(long long)(t + TL * j) * xstride] : mk<C2>(0, 0);
+    for (int i = threadIdx.x; i < N; i += blockDim.x) tw[i] = twx[i];
+    const bool grad = op.kind == GREEN_TGRAD;
+    const T fz = (T)sfreq(kz, op.pos_nyq ? g.Nz / 2 : (g.Nz - 1) / 2, g.Nz);
+    const T fy = (T)sfreq(y, op.pos_nyq ? g.Ny / 2 : (g.Ny - 1) / 2, g.Ny);
+    const bool origin = ok && y == 0 && kz == 0;
+    __syncthreads();
+    line_fwd<C2, E, TL>(v, t, xl, tw, sw);
+    const C2 k0 = mk<C2>(__shfl_sync(0xffffffffu, v[0].x, col), __shfl_sync(0xffffffffu, v[0].y, col));  // t = 0: mode 0
+#pragma unroll
+    for (int r = 0; r < E; ++r) modes[(c * E + r) * 32 + lane] = v[r];
+    __syncthreads();
+#pragma unroll
+    for (int r = 0; r < E; ++r) {
+        const int mode = spec_mode<E, TL>(t, r);
+        const T fx = (T)sfreq(mode, op.pos_nyq ? g.Nx / 2 : (g.Nx - 1) / 2, op.xwrap);
+        C2 d = mk<C2>(0, 0);
+#pragma unroll
+        for (int q = 0; q < C; ++q) {
+            const C2 m = modes[(q * E + r) * 32 + lane];
+            const T fc = q == 2 ? fx : (q == 0 ? fz : fy);
+            d = r1_add(d, fc, m);
+        }
+        const T n2 = r1_norm2(fz, fy, fx);
+        const T coef = (origin && mode == 0) ? (T)0 : (grad ? -op.p1 : (T)1) / n2;
+        d = r1_scale(coef, d);
+        v[r] = c == 2 ? r1_scale(fx, d) : d;
+    }
+    C2 add = mk<C2>(0, 0);
+    if (origin) {
+        const T kc = op.zero_k0 ? (T)0 : (T)ctl[b].kzero[c];
+        add = grad ? mk<C2>(kc, 0) : r1_add(mk<C2>(kc, 0), op.p1, k0);
+    }
+    const T sc = grad ? (T)1 : op.p1;
+    const T f = c == 2 ? (T)1 : (c == 0 ? fz : fy);
+    line_inv<C2, E, TL>(v, t, xl, tw, sw);
+    if (!ok) return;
+#pragma unroll
+    for (int j = 0; j < E; ++j) {
+        C2* p = base + (long long)(t + TL * j) * xstride;
+        C2 o = r1_scale(sc * f, v[j]);
+        if (!grad) o = r1_add(o, -(op.p1 * (T)N), *p);
+        *p = r1_add(o, (T)1, add);
+    }
 }
 
 // ---------------------------------------------------------------------------
@@ -701,7 +795,7 @@ __global__ void __launch_bounds__(32 * kXRegWarps, XR1TmaMinB<T, N>::value)
 #pragma unroll
             for (int r = 0; r < E; ++r) {
                 const T fc = c == 2 ? fx[r] : fcol;
-                d[r] = mk<C2>(d[r].x + fc * v[r].x, d[r].y + fc * v[r].y);
+                d[r] = r1_add(d[r], fc, v[r]);
             }
         }
         if (failed) {
@@ -712,17 +806,17 @@ __global__ void __launch_bounds__(32 * kXRegWarps, XR1TmaMinB<T, N>::value)
 #pragma unroll
         for (int r = 0; r < E; ++r) {
             const int mode = spec_mode<E, TL>(t, r);
-            const T n2 = fz * fz + fy * fy + fx[r] * fx[r];
+            const T n2 = r1_norm2(fz, fy, fx[r]);
             const T coef = (origin && mode == 0) ? (T)0 : (grad ? -op.p1 : (T)1) / n2;
-            d[r] = mk<C2>(coef * d[r].x, coef * d[r].y);
-            v[r] = mk<C2>(fx[r] * d[r].x, fx[r] * d[r].y);
+            d[r] = r1_scale(coef, d[r]);
+            v[r] = r1_scale(fx[r], d[r]);
         }
         C2 add[C] = {mk<C2>(0, 0), mk<C2>(0, 0), mk<C2>(0, 0)};
         if (origin) {
 #pragma unroll
             for (int c = 0; c < C; ++c) {
                 const T kc = op.zero_k0 ? (T)0 : (T)ctl[b].kzero[c];
-                add[c] = grad ? mk<C2>(kc, 0) : mk<C2>(kc + op.p1 * k0[c].x, op.p1 * k0[c].y);
+                add[c] = grad ? mk<C2>(kc, 0) : r1_add(mk<C2>(kc, 0), op.p1, k0[c]);
             }
         }
         const T sc = grad ? (T)1 : op.p1;
@@ -730,12 +824,9 @@ __global__ void __launch_bounds__(32 * kXRegWarps, XR1TmaMinB<T, N>::value)
 #pragma unroll
             for (int j = 0; j < E; ++j) {
                 C2* p = base + c * cstride + (long long)(t + TL * j) * xstride;
-                C2 o = mk<C2>(sc * f * u[j].x, sc * f * u[j].y);
-                if (!grad) {
-                    const C2 in = *p;
-                    o = mk<C2>(o.x - op.p1 * (T)N * in.x, o.y - op.p1 * (T)N * in.y);
-                }
-                *p = mk<C2>(o.x + add[c].x, o.y + add[c].y);
+                C2 o = r1_scale(sc * f, u[j]);
+                if (!grad) o = r1_add(o, -(op.p1 * (T)N), *p);
+                *p = r1_add(o, (T)1, add[c]);
             }
         };
         line_inv<C2, E, TL>(d, t, xl, tw, sw);

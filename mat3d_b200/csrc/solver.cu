@@ -740,20 +740,27 @@ int m3d_solver::pass_x(Spec op, Ctl* ctl, typename Cx<T>::t* sp) {
     const bool done = use_fast && with_fast_n(Nx, [&](auto nc) {
         constexpr int NN = decltype(nc)::value;
         constexpr int CPW = 32 / LineSplit<T, NN>::Tl;
-        // The rank-one form gives a warp a column group of all three components, one
-        // after the other; with few of them that chain is the pass's time, and a warp
-        // per component is faster although it transforms three inverses where the
-        // rank-one form transforms two.  A solve took, by column groups of the batch
-        // (rank-one -> by component, ms): FP64 96 (32^3, one entry) 0.96 -> 0.87,
-        // 288 1.02 -> 0.93, 576 (64^3) 1.39 -> 1.36, 864 1.70 -> 1.77, 1728 1.92 -> 2.15;
-        // FP32 sweeps 96 1.44 -> 1.29, 576 1.70 -> 1.63, 672 (96^3) 3.29 -> 3.21,
-        // 1728 2.32 -> 2.42.  At 16 points the two are equal.
-        const bool few = CC == 3 && use_xcp && NN >= 32 && (long long)B * Ny * ((g.Hzp + CPW - 1) / CPW) <= 5 * 148;
         // (not FP64 at N = 96: its 24 points per lane spill at any register cap)
         if constexpr (CC == 3 && NN <= 128 && (sizeof(T) == 4 || NN != 96) &&
                       std::is_same<Spec, SpecGreen<T, 3>>::value) {
-            if (use_xr1 && !few) {  // thermal Green operators in rank-one form; warp-granular (y, column group) items
+            if (use_xr1) {  // thermal Green operators in rank-one form; warp-granular (y, column group) items
                 const int ngrp = (g.Hzp + CPW - 1) / CPW;
+                // With few column groups the chain of a warp that does all three
+                // components is the pass's time, and a warp per component is faster
+                // although it transforms one line more.  Solves, by column groups
+                // of the batch: FP64 96 (32^3) 0.96 -> 0.82 ms, 192 (48^3) 1.22 -> 1.05,
+                // 576 (64^3) 1.35 -> 1.27; FP32 sweeps 96 1.41 -> 1.21, 576 1.73 -> 1.63,
+                // 672 (96^3) 3.40 -> 3.31.  Five groups an SM: at 864 groups and above
+                // the warps of k_xturn_r1 fill the chip (the six-transform kernel, ahead
+                // by 2% at 576, was behind by 4% at 864 and 10% at 1728).
+                if constexpr (NN <= 96) {
+                    if (use_xcp && NN >= 32 && (long long)B * Ny * ngrp <= 5 * 148) {
+                        nblk = Ny * ngrp;
+                        allow_smem(k_xturn_r1cp<T, NN>);
+                        k_xturn_r1cp<T, NN><<<dim3(nblk, gridB()), 96, xturn_r1cp_smem<T, NN>(), stream>>>(g, tw<T>(0), sp, op, ctl);
+                        return;
+                    }
+                }
                 if constexpr (sizeof(T) == 4) {
                     if (use_xr1_tma && (void*)sp == d_spec && ensure_xmap(CPW)) {  // column loads staged by TMA
                         typedef XR1Tma<T, NN> X;
@@ -782,7 +789,7 @@ int m3d_solver::pass_x(Spec op, Ctl* ctl, typename Cx<T>::t* sp) {
             }
         }
         if constexpr (CC == 3 && sizeof(T) == 4 && NN <= 64) {
-            if (use_xreg && !few) {  // the three components in registers (fits them without spilling up to N = 64)
+            if (use_xreg) {  // the three components in registers (fits them without spilling up to N = 64)
                 const int ntz = (g.Hzp + kXRegWarps * CPW - 1) / (kXRegWarps * CPW);
                 nblk = Ny * ntz;
                 allow_smem(k_xturn_reg<T, NN, Spec>);

@@ -1,10 +1,11 @@
 """The thermal x turnaround of few column groups (a warp per component,
-`k_xturn_cp`) against the rank-one and register kernels (`M3D_XTURN_CP=0`), on
-grids and batches on both sides of the rule's line (740 groups), in each precision
-and both stop rules.  Per mode the two differ by the rounding of a dozen
-operations, at most a few 1e-7 of the field in FP32 and 1e-15 in FP64 a sweep, and
-a converging sweep damps what the one before left: rel-L2 below 1e-5 for FP32
-sweeps (1e-9 with refinement, which solves to 1e-10) and 1e-12 for FP64.
+`k_xturn_r1cp`) against the kernel that gives a warp all three
+(`M3D_XTURN_CP=0`), on grids and batches on both sides of the rule's line (740
+groups), in each precision.  Under the residual rule both do the same arithmetic:
+equal bits and sweep counts, also of an entry alone and the same entry in a batch
+of the other kernel.  Under the reference rule the switch picks other kernels,
+which sum the check in another order: the fields agree to rounding, rel-L2 below
+1e-5 in FP32 and 1e-12 in FP64.
 Reference: src/3dTherm/FFT_thermal3D.cpp:200-266."""
 import numpy as np
 import pytest
@@ -42,4 +43,25 @@ def test_few_columns(N, nrve, prec, tol, bound, criterion, monkeypatch):
             out.append((s.stats()["sweeps"], C))
         s.close()
     assert out[0][0] == out[1][0]
+    if criterion == m3d.CRIT_RESIDUAL:
+        assert np.array_equal(out[0][1], out[1][1])
     assert rel(out[0][1], out[1][1]) < bound
+
+
+@pytest.mark.parametrize("prec,tol", [("fp32", 1e-4), ("fp32_refine", 1e-9), ("fp64", 1e-6)])
+@pytest.mark.parametrize("contrast", [12.0, 0.08])  # gradient- and flux-based
+def test_entry_alone_and_in_a_batch(contrast, prec, tol):
+    N, nrve = 32, 9  # 96 and 864 column groups
+    rng = np.random.default_rng(5)
+    rve = (rng.random((nrve, N ** 3)) < 0.3).astype(np.int32)
+    E = np.array([0.01, 0.003, -0.002])
+    fields = []
+    for which in (range(nrve), [4]):
+        s = m3d.Solver(m3d.KIND_THERMAL, N, N, N, m3d.ELASTIC, prec, nrve=len(which), nload=1)
+        for i, r in enumerate(which):
+            s.set_material_thermal(1.0, contrast, rve[r], rve=i)
+            s.set_load(E, b=i)
+        s.run(tol, tol, 1, m3d.CRIT_RESIDUAL)
+        fields.append(s.field(m3d.FIELD_STRAIN, list(which).index(4)))
+        s.close()
+    assert np.array_equal(*fields)
