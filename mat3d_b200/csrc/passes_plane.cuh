@@ -38,7 +38,7 @@
 // k_zmid runs at the memory bandwidth from 48^3 on; k_plane is bound by the
 // shared-memory pipe (67% busy at 96^3: 16 accesses of a point in shared
 // memory, the rows' global accesses in 32-byte pieces) and by issue (45%).
-// FP64 96^3 (147 KB a component) keeps the five passes.
+// FP64 96^3 (147 KB a component) has the four passes of passes_zmid.cuh.
 #pragma once
 #include <cooperative_groups.h>
 
