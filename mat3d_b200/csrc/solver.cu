@@ -328,9 +328,14 @@ struct m3d_solver {
     template <typename T, int CC> bool mid_ok() const;
     // sweeps whose last kernel also does the next sweep's z forward
     template <typename T, int CC> bool fused_ok() const { return two_pass_ok<T, CC>() || mid_ok<T, CC>(); }
-    template <typename T, int CC> int launches_per_sweep(bool fused) const {
-        return !fused ? 5 : (two_pass_ok<T, CC>() ? 2 : 4);
+    // the sweep a solve runs, by shape and material: separate passes, slab, plane
+    // or fused z pass
+    enum Sweep { SWEEP_FIVE = 0, SWEEP_SLAB = 1, SWEEP_PLANE = 2, SWEEP_FOUR = 3 };
+    template <typename T, int CC> Sweep sweep_kind(bool fused) const {
+        if (!fused) return SWEEP_FIVE;
+        return plane_ok<T, CC>() ? SWEEP_PLANE : (slab_ok<T>() ? SWEEP_SLAB : SWEEP_FOUR);
     }
+    static int launches_per_sweep(Sweep k) { return k == SWEEP_FIVE ? 5 : (k == SWEEP_FOUR ? 4 : 2); }
     template <typename T, class Op, class Fin>
     int pass_zmid_gen(const typename Op::Args& op, Ctl* ctl, typename Cx<T>::t* sp, const Fin& fin);
     template <typename T> int pass_zmid_inelastic(const MidJ2Args& op, Ctl* ctl, typename Cx<T>::t* sp, const FinJ2& fin);
@@ -388,9 +393,12 @@ struct m3d_solver {
             s.key = -1;
         }
     }
-    long long graph_key(int type) const {
-        return (((((long long)type * 8192 + B) * 32 + nph_max()) * 2 + (use_fast ? 1 : 0)) * 4 + prec) * 2 +
-               (use_slab ? 1 : 0);
+    // What a captured graph depends on.  The sweep is part of it: a material
+    // change may make the operators diagonal or couple them, and the sweeps keep
+    // the half spectrum in different layouts between their passes.
+    long long graph_key(int type, Sweep sweep) const {
+        return ((((((long long)type * 8192 + B) * 32 + nph_max()) * 2 + (use_fast ? 1 : 0)) * 4 + prec) * 2 +
+                (use_slab ? 1 : 0)) * 4 + sweep;
     }
     template <typename T, int CC>
     int run_linear_graph(double tol_field, double tol_eq, int criterion, int max_iter);
@@ -1060,7 +1068,7 @@ int m3d_solver::run_linear(double tol_field, double tol_eq, int criterion, int m
     const int chunk = kChunk;
     int before = 0;
     const bool slab = criterion == M3D_CRIT_RESIDUAL && fused_ok<T, CC>();
-    st.passes_per_sweep = launches_per_sweep<T, CC>(slab);
+    st.passes_per_sweep = launches_per_sweep(sweep_kind<T, CC>(slab));
     if (slab) {
         rc = pass_slab<T, CC, false>(d_ctl, x, nullptr, sp, FinNone{});
         if (rc) return rc;
@@ -1121,7 +1129,7 @@ int m3d_solver::run_refine(double tol_field, int max_iter) {
     bool first = true;
     const int chunk = 8;
     const bool slab = fused_ok<float, CC>();
-    st.passes_per_sweep = launches_per_sweep<float, CC>(slab);
+    st.passes_per_sweep = launches_per_sweep(sweep_kind<float, CC>(slab));
     std::vector<long long> in32((size_t)B, 0);  // FP32 sweeps per entry
     for (;;) {
         ProRefine64<CC> pro = tab(ProRefine64<CC>{d_phase, x, first ? nullptr : d_delta, g.V, dm(off_P), nph_max(), nullptr});
@@ -1365,13 +1373,14 @@ int m3d_solver::run_linear_graph(double tol_field, double tol_eq, int criterion,
     M3D_CUDA(cudaMemsetAsync(d_trips, 0, 8 * sizeof(int), stream));
     const bool resid = (criterion == M3D_CRIT_RESIDUAL);
     const bool slab = resid && fused_ok<T, CC>();
-    st.passes_per_sweep = launches_per_sweep<T, CC>(slab);
+    const Sweep kind_of_sweep = sweep_kind<T, CC>(slab);
+    st.passes_per_sweep = launches_per_sweep(kind_of_sweep);
     if (slab) {
         rc = pass_slab<T, CC, false>(d_ctl, x, nullptr, sp, FinNone{});
         if (rc) return rc;
     }
     GraphSlot& gs = gslot[resid ? 0 : 1];
-    const long long key = graph_key(resid ? 0 : 1);
+    const long long key = graph_key(resid ? 0 : 1, kind_of_sweep);
     const std::vector<int> lv = resid ? compact_levels() : std::vector<int>();
     if (gs.key != key) {
         drop_graphs();
@@ -1465,10 +1474,11 @@ int m3d_solver::run_refine_graph(double tol_field, int max_iter) {
     M3D_CUDA(cudaMemsetAsync(d_ctl_in, 0, (size_t)B * sizeof(Ctl), stream));
     M3D_CUDA(cudaMemsetAsync(d_trips, 0, 8 * sizeof(int), stream));
     const bool slab = fused_ok<float, CC>();
-    st.passes_per_sweep = launches_per_sweep<float, CC>(slab);
+    const Sweep kind_of_sweep = sweep_kind<float, CC>(slab);
+    st.passes_per_sweep = launches_per_sweep(kind_of_sweep);
     const size_t sbytes32 = (size_t)B * CC * g.NL * g.Hzp * sizeof(float2);
     GraphSlot& gs = gslot[2];
-    const long long key = graph_key(2);
+    const long long key = graph_key(2, kind_of_sweep);
     const std::vector<int> lv = compact_levels();  // levels of the compacted inner loop (none: one loop)
     if (gs.key != key) {
         drop_graphs();
