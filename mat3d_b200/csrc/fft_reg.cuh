@@ -75,9 +75,11 @@ M3D_SPLIT(double, 128, 16, 8)
 M3D_SPLIT(double, 256, 16, 16)
 #undef M3D_SPLIT
 
-constexpr bool fast_size(int n) {
-    return n == 16 || n == 32 || n == 48 || n == 64 || n == 96 || n == 128 || n == 256;
-}
+// line lengths with compile-time passes
+constexpr bool fast_line(int n) { return n == 32 || n == 48 || n == 64 || n == 96 || n == 128 || n == 256; }
+// grid lengths whose schedules the autotuner takes as they are: 16 points are a
+// single radix-16 stage, with no order or tile to choose
+constexpr bool fast_size(int n) { return n == 16 || fast_line(n); }
 
 // exchange buffer of one line: element (k1, t) at k1*(T+1) + t
 template <int E, int T> struct Xch { static constexpr int size = E * (T + 1) + 1; };

@@ -937,12 +937,15 @@ bool m3d_solver::plane_ok() const {
 
 // Other shapes: the fused z pass on the row layout (passes_zmid.cuh), four launches
 // a sweep: y forward, x turnaround, y inverse, z inverse + update + z forward.
-// Compile-time lengths up to 96 that the two-pass sweeps leave (non-cubic grids)
-// keep five passes.
+// Lines without a compile-time transform all have it (16 points among them: elastic
+// FP64 16^3 1.02 ms a solve with five passes, 0.82 with four).  Compile-time lines have
+// it at 96 points in FP64 and above; shorter ones that the two-pass sweeps leave
+// (non-cubic grids) keep five passes, and so do thermal FP32 lines of 128 points
+// on grids whose y length differs.
 template <typename T, int CC>
 bool m3d_solver::mid_ok() const {
     if (!use_slab) return false;
-    if (!(use_fast && fast_size(Nz))) return true;
+    if (!(use_fast && fast_line(Nz))) return true;
     return (Nz > 96 || (Nz == 96 && sizeof(T) == 8)) && zmid_rows_ok<T>(Nz, CC, g.NL);
 }
 
@@ -960,7 +963,7 @@ int m3d_solver::pass_zmid_gen(const typename Op::Args& op, Ctl* ctl, typename Cx
 template <typename T>
 int m3d_solver::pass_zmid_inelastic(const MidJ2Args& op, Ctl* ctl, typename Cx<T>::t* sp, const FinJ2& fin) {
     const bool j2 = behav == M3D_BEHAV_J2;
-    if (!(use_fast && fast_size(Nz)))
+    if (!(use_fast && fast_line(Nz)))
         return j2 ? pass_zmid_gen<T, MidJ2<T, true>>(op, ctl, sp, fin) : pass_zmid_gen<T, MidJ2<T, false>>(op, ctl, sp, fin);
     M3D_CUDA(zmid_rows_inelastic<T>(Nz, j2, gridB(), stream, g, tw<T>(2), sp, op, ctl, d_part, fin));
     st.kernel_launches += 1;
@@ -972,7 +975,7 @@ int m3d_solver::pass_slab(Ctl* ctl, T* x, const float* r, typename Cx<T>::t* sp,
     if (!two_pass_ok<T, CC>()) {
         if constexpr (MIX) {
             const MidEMArgs<T> op = tab(MidEMArgs<T>{d_phase, x, r, g.V, dm(off_P), dm(off_A), nph_max()});
-            if (!(use_fast && fast_size(Nz))) return pass_zmid_gen<T, MidEM<T, 1, CC>>(op, ctl, sp, fin);
+            if (!(use_fast && fast_line(Nz))) return pass_zmid_gen<T, MidEM<T, 1, CC>>(op, ctl, sp, fin);
             M3D_CUDA(zmid_rows_em<T>(Nz, CC, gridB(), stream, g, tw<T>(2), sp, op, ctl, d_part, fin));
             st.kernel_launches += 1;
         } else {

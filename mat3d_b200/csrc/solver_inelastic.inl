@@ -182,7 +182,7 @@ int m3d_solver::run_inelastic(double tol_field, double tol_eq, int nInc, int cri
     SpecBasic<T> spec{green<T, 6>(0), SpecEqVar<T, 6>{g}};
     // fused z pass (z inverse, update, next z forward): every length but the
     // compile-time ones whose tiles the lines do not fill; the stress then stays in registers and is written at the end of an increment
-    const bool mid = use_slab && (!(use_fast && fast_size(Nz)) || zmid_rows_ok<T>(Nz, 6, g.NL));
+    const bool mid = use_slab && (!(use_fast && fast_line(Nz)) || zmid_rows_ok<T>(Nz, 6, g.NL));
     st.passes_per_sweep = mid ? 4 : 5;
     const MidJ2Args margs{d_phase, eps, eps_old, sig_old, ep, dmg, V, in.d_ph, nph, pro.sig_old ? 1 : 0, in.d_nrfail};
     // the convergence sums of the stress spectrum are the reference rule's alone

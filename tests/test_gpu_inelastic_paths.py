@@ -40,7 +40,7 @@ def solve(shape, behav, prec, crit, fused, monkeypatch):
 @pytest.mark.parametrize("prec,bound", [("fp64", 1e-11), ("fp32", 1e-5)])
 @pytest.mark.parametrize("crit", [m3d.CRIT_REFERENCE, m3d.CRIT_RESIDUAL])
 @pytest.mark.parametrize("behav", [m3d.J2, m3d.DAMAGE])
-@pytest.mark.parametrize("shape", [(7, 9, 25), (5, 7, 26), (6, 5, 38)])
+@pytest.mark.parametrize("shape", [(7, 9, 25), (5, 7, 26), (6, 5, 38), (16, 16, 16)])
 def test_generic_lines_match_separate_passes(shape, behav, crit, prec, bound, monkeypatch):
     a, sa = solve(shape, behav, prec, crit, True, monkeypatch)
     b, sb = solve(shape, behav, prec, crit, False, monkeypatch)
@@ -73,11 +73,13 @@ def linear(kind, shape, prec, fused, monkeypatch):
     return f, st
 
 
+# FP64 and FP32 fields: the same sums in another order; refined ones stop at a residual of 1e-9
 @pytest.mark.parametrize("kind,shape,prec", [(m3d.KIND_THERMAL, (6, 8, 128), "fp64"), (m3d.KIND_THERMAL, (4, 8, 96), "fp64"),
-                                             (m3d.KIND_MECH, (4, 8, 96), "fp64")])
+                                             (m3d.KIND_MECH, (4, 8, 96), "fp64")] +
+                         [(k, (16, 16, 16), p) for k in (m3d.KIND_THERMAL, m3d.KIND_MECH) for p in ("fp64", "fp32", "fp32_refine")])
 def test_linear_fused_pass(kind, shape, prec, monkeypatch):
     a, sa = linear(kind, shape, prec, True, monkeypatch)
     b, sb = linear(kind, shape, prec, False, monkeypatch)
     assert (sa["passes_per_sweep"], sb["passes_per_sweep"]) == (4, 5)
-    assert sa["sweeps"] == sb["sweeps"]
-    assert rel(a, b) < 1e-10
+    assert sa["sweeps_fp64"] == sb["sweeps_fp64"] and abs(sa["sweeps_fp32"] - sb["sweeps_fp32"]) <= 2
+    assert rel(a, b) < {"fp64": 1e-10, "fp32": 1e-5, "fp32_refine": 1e-8}[prec]
