@@ -12,36 +12,12 @@
 // The radix-13 and radix-31 variants are instantiated in generic_r13.cu and
 // generic_r31.cu, compiled beside solver.cu.
 #pragma once
-#include <mutex>
-#include <set>
-#include <utility>
-
 #include "inelastic.cuh"
 #include "passes.cuh"
 #include "physics.cuh"
+#include "smem_limit.cuh"
 
 namespace m3d {
-
-// Let a kernel use all dynamic shared memory left next to its static arrays
-// (227 KB per block on sm_100 in total).
-// Done once per kernel and device; safe to call from several host threads.
-inline std::mutex g_attr_mu;
-inline std::set<std::pair<int, const void*>> g_attr_done;
-template <class K>
-void allow_smem(K kernel) {
-    int dev = 0;
-    cudaGetDevice(&dev);
-    {
-        std::lock_guard<std::mutex> lk(g_attr_mu);
-        if (!g_attr_done.insert(std::make_pair(dev, (const void*)kernel)).second) return;
-    }
-    cudaFuncAttributes a;
-    if (cudaFuncGetAttributes(&a, kernel) == cudaSuccess) {
-        const int maxdyn = 227 * 1024 - (int)a.sharedSizeBytes;
-        cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, maxdyn);
-    }
-    (void)cudaGetLastError();  // an unsupported request must not surface at the next launch check
-}
 
 // The variant of a plan: the smallest that holds its odd radices (primes up to 31).
 inline int max_radix(const LinePlan& p) {

@@ -1,6 +1,6 @@
 // plane.cu -- kernels and launches of the two-pass elastic sweep.
-#include "generic_launch.cuh"  // allow_smem
 #include "plane_launch.cuh"
+#include "smem_limit.cuh"
 
 namespace m3d {
 
