@@ -217,9 +217,46 @@ __device__ __forceinline__ void dft_small(C2 (&v)[R], const C2* tw, int n, int s
         v[4] = mk<C2>(t1.x + u1.y, t1.y - u1.x);
         v[2] = mk<C2>(t2.x - u2.y, t2.y + u2.x);
         v[3] = mk<C2>(t2.x + u2.y, t2.y - u2.x);
-    } else if constexpr (R == 9 || R == 16) {
-        // R = P x P: w_R twiddles between two rounds of P-point DFTs
-        constexpr int P = R == 9 ? 3 : 4;
+    } else if constexpr (R == 9) {
+        // inputs m and 9 - m paired (see butterfly_odd): about the operations of two
+        // rounds of 3-point DFTs with w_9 twiddles between them, which rounded more
+        // (FP64 transforms of 27, 81, 171 and 729 points 4, 10, 9 and 19% further from
+        // their exact values); solves at lengths of nines take 0 to 2% longer
+        const T cs[9] = {(T)1, (T)0.766044443118978035202392650555417L, (T)0.173648177666930348851716626769315L, (T)-0.5,
+                         (T)-0.939692620785908384054109277324731L, (T)-0.939692620785908384054109277324731L, (T)-0.5,
+                         (T)0.173648177666930348851716626769315L, (T)0.766044443118978035202392650555417L};
+        const T sn[9] = {(T)0, (T)0.642787609686539326322643409907263L, (T)0.984807753012208059366743024589523L,
+                         (T)0.866025403784438646763723170752936L, (T)0.342020143325668733044099614682260L,
+                         (T)-0.342020143325668733044099614682260L, (T)-0.866025403784438646763723170752936L,
+                         (T)-0.984807753012208059366743024589523L, (T)-0.642787609686539326322643409907263L};
+        C2 a[4], b[4], out[8];
+        C2 sum = v[0];
+#pragma unroll
+        for (int m = 1; m < 5; ++m) {
+            a[m - 1] = cadd(v[m], v[9 - m]);
+            b[m - 1] = csub(v[m], v[9 - m]);
+            sum = cadd(sum, a[m - 1]);
+        }
+#pragma unroll
+        for (int k = 1; k < 5; ++k) {
+            C2 A = v[0], B = mk<C2>(0, 0);
+#pragma unroll
+            for (int m = 1; m < 5; ++m) {
+                const T c = cs[k * m % 9], d = sign < 0 ? -sn[k * m % 9] : sn[k * m % 9];
+                A.x += c * a[m - 1].x;
+                A.y += c * a[m - 1].y;
+                B.x += d * b[m - 1].x;
+                B.y += d * b[m - 1].y;
+            }
+            out[k - 1] = mk<C2>(A.x - B.y, A.y + B.x);
+            out[8 - k] = mk<C2>(A.x + B.y, A.y - B.x);
+        }
+        v[0] = sum;
+#pragma unroll
+        for (int k = 1; k < 9; ++k) v[k] = out[k - 1];
+    } else if constexpr (R == 16) {
+        // 4 x 4: w_16 twiddles between two rounds of 4-point DFTs
+        constexpr int P = 4;
         C2 sub[P][P];
 #pragma unroll
         for (int p = 0; p < P; ++p) {
@@ -231,21 +268,7 @@ __device__ __forceinline__ void dft_small(C2 (&v)[R], const C2* tw, int n, int s
         for (int k1 = 0; k1 < P; ++k1) {
             C2 t[P];
 #pragma unroll
-            for (int p = 0; p < P; ++p) {
-                if (p == 0 || k1 == 0) {
-                    t[p] = sub[p][k1];
-                } else if constexpr (R == 16) {
-                    t[p] = rot_const<C2, 16>(sub[p][k1], p * k1, sign);
-                } else {  // cos and sin of 40, 80 and 160 degrees
-                    const T c = p * k1 == 1 ? (T)0.766044443118978035202392650555417L
-                                            : (p * k1 == 2 ? (T)0.173648177666930348851716626769315L
-                                                           : (T)-0.939692620785908384054109277324731L);
-                    const T sn = p * k1 == 1 ? (T)0.642787609686539326322643409907263L
-                                             : (p * k1 == 2 ? (T)0.984807753012208059366743024589523L
-                                                            : (T)0.342020143325668733044099614682260L);
-                    t[p] = cmul(sub[p][k1], mk<C2>(c, sign < 0 ? -sn : sn));
-                }
-            }
+            for (int p = 0; p < P; ++p) t[p] = p == 0 || k1 == 0 ? sub[p][k1] : rot_const<C2, 16>(sub[p][k1], p * k1, sign);
             dft_small<C2, P>(t, tw, n, sign);
 #pragma unroll
             for (int k2 = 0; k2 < P; ++k2) v[k1 + P * k2] = t[k2];
