@@ -19,6 +19,11 @@ LIB = os.path.join(HERE, "libmat3d_b200.so")
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a",
     "-O3", "-lineinfo", "-std=c++17",
+    # The line tables are three quarters of the device images, and a compressed image
+    # is unpacked whole when a process first uses one of its kernels, at about 1 GB/s.
+    # From a fresh process, handle and first solve: thermal FP64 65^3 83 -> 49 ms, FP64
+    # 32^3 65 -> 35, elastic FP32 + refinement 75^3 86 -> 46.  (The library is 163 MB, not 62.)
+    "--compress-mode=none",
     "-Xcompiler", "-fPIC", "-shared", "--threads", "0",  # one compiler per source at a time
 ]
 
