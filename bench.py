@@ -61,34 +61,51 @@ def bytes_per_vi(c, w):
     return 6 * c * w + 1
 
 
-PASS_NAMES = ("z_forward", "y_forward", "x_turnaround", "y_inverse", "z_inverse")
-PASS_KERNELS = ("k_zfwd_fast (prologue + z R2C)", "k_ypass_fast<-1>", "k_xturn_fast (x FFT, Green, x IFFT)",
-                "k_ypass_fast<+1>", "k_zinv_fast (z C2R + EM update + finalize)")
-# two-pass sweeps (per-component operators): the profile's slot 2 is the x
-# turnaround, slot 4 the y-z slab pass, the other slots are empty
-PASS_NAMES_2 = (None, None, "x_turnaround", None, "yz_slab")
-PASS_KERNELS_2 = (None, None, "k_xturn_fast (x FFT, Green, x IFFT)", None,
-                  "k_slab<MIX> (y IFFT, z C2R, EM update, polarization, z R2C, y FFT + finalize)")
+# The profile's five slots by the sweep that ran (m3d_stats.passes_per_sweep and, of
+# two passes, the physics): what each launch is called and which kernel it is.  Slots
+# without a launch are None.
+SWEEP_PASSES = {
+    "five": (("z_forward", "k_zfwd_fast (prologue + z R2C)"), ("y_forward", "k_ypass_fast<-1>"),
+             ("x_turnaround", "k_xturn_* (x FFT, Green, x IFFT)"), ("y_inverse", "k_ypass_fast<+1>"),
+             ("z_inverse", "k_zinv_fast (z C2R + EM update + finalize)")),
+    "four": (None, ("y_forward", "k_ypass_fast<-1>"), ("x_turnaround", "k_xturn_* (x FFT, Green, x IFFT)"),
+             ("y_inverse", "k_ypass_fast<+1>"),
+             ("z_fused", "k_zmid_rows (z C2R, update, z R2C + finalize)")),
+    "slab": (None, None, ("x_turnaround", "k_xturn_* (x FFT, Green, x IFFT)"), None,
+             ("yz_slab", "k_slab<MIX> (y IFFT, z C2R, EM update, polarization, z R2C, y FFT + finalize)")),
+    "plane": (None, None, ("kz_plane", "k_plane (y FFT, x FFT, Green, x IFFT, y IFFT)"), None,
+              ("z_fused", "k_zmid (z C2R, EM update, polarization, z R2C + finalize)")),
+}
 
 
-def pass_bytes(c, w, N, forcing, two_pass=False):
-    """Algorithmic bytes per launch of each sweep pass on an N^3 grid with c
-    components of w-byte reals: the pass's own inputs and outputs (half
-    spectrum N*N*Hzp complex per component, Hzp = N/2+1 rounded up to even;
-    state c*V reals; 1-byte phase; the FP32 defect read by the refinement's
-    inner sweeps).  Two-pass sweeps: the x turnaround, and the slab pass that
-    reads and writes the spectrum and the state once, reads the defect and the
-    phase map once per component."""
+def sweep_of(passes, kind):
+    """Key of SWEEP_PASSES for a run's passes_per_sweep: of the two-pass sweeps the
+    elastic operators, which couple the components, have the kz-plane one."""
+    return {5: "five", 4: "four", 2: "slab" if kind == "thermal" else "plane"}[passes]
+
+
+def pass_names(sweep):
+    return [p[0] if p else None for p in SWEEP_PASSES[sweep]]
+
+
+def pass_bytes(c, w, N, forcing, sweep="five"):
+    """Algorithmic bytes per launch of each slot on an N^3 grid with c components of
+    w-byte reals: the pass's own inputs and outputs (half spectrum N*N*Hzp complex per
+    component, Hzp = N/2+1 rounded up to even, of the kz-plane sweep N/2+1; state c*V
+    reals; 1-byte phase; the FP32 defect read by the refinement's inner sweeps).  A
+    fused last pass reads and writes the spectrum and the state once; the slab pass,
+    which takes one component at a time, reads the phase map once per component."""
     V = N ** 3
-    hzp = ((N // 2 + 1) + 1) & ~1
-    spec = c * N * N * hzp * 2 * w
+    hz = N // 2 + 1
+    spec = c * N * N * (hz if sweep == "plane" else (hz + 1) & ~1) * 2 * w
     state = c * V * w
     forcing_b = c * V * 4 if forcing else 0
-    if two_pass:
-        return (0, 0, 2 * spec, 0, 2 * spec + 2 * state + c * V + forcing_b)
-    zfwd = state + V + spec
-    zinv = spec + 2 * state + V + forcing_b
-    return (zfwd, 2 * spec, 2 * spec, 2 * spec, zinv)
+    fused = 2 * spec + 2 * state + (c * V if sweep == "slab" else V) + forcing_b
+    if sweep == "five":
+        return (state + V + spec, 2 * spec, 2 * spec, 2 * spec, spec + 2 * state + V + forcing_b)
+    if sweep == "four":
+        return (0, 2 * spec, 2 * spec, 2 * spec, fused)
+    return (0, 0, 2 * spec, 0, fused)
 
 
 # DRAM bytes per launch (dram__bytes_read.sum + dram__bytes_write.sum) from
@@ -921,7 +938,6 @@ def profile_batch_groups(args, w):
     sweeps."""
     import mat3d_b200 as m3d
     from mat3d_b200 import rve as R
-    names = ["z_forward", "y_forward", "x_turnaround", "y_inverse", "z_inverse"]
     desc = R.batch_rves(EXTRA_BATCH_COUNT)
     groups = {}
     for d in desc:
@@ -936,12 +952,15 @@ def profile_batch_groups(args, w):
         s.homogenize(w["tol"])
         p, st = s.profile(), s.stats()
         r = {"rves": len(ds), "entries": 6 * len(ds), "entry_sweeps_fp32": st["sweeps_fp32"],
-             "entry_sweeps_fp64": st["sweeps_fp64"]}
+             "entry_sweeps_fp64": st["sweeps_fp64"], "passes_per_sweep": st["passes_per_sweep"]}
+        fp32_names = pass_names(sweep_of(st["passes_per_sweep"], "mech"))
         for tag in ("fp32", "fp64"):
             if p[f"n_{tag}"]:
                 r[f"trips_{tag}"] = p[f"n_{tag}"]
                 r[f"ms_{tag}"] = p[f"ms_{tag}"]
-                r[f"pass_ms_{tag}"] = {names[q]: p[f"pass_ms_{tag}"][q] for q in range(5)}
+                # the refinement's FP64 defect sweeps run the five passes
+                nm = fp32_names if tag == "fp32" else pass_names("five")
+                r[f"pass_ms_{tag}"] = {nm[q]: p[f"pass_ms_{tag}"][q] for q in range(5) if nm[q]}
         out["groups"][N] = r
         s.close()
     return out
@@ -967,7 +986,7 @@ def profile_passes(args, w):
         s.set_load(E, X0)
         s.run(w["tol"], w["tol"], w.get("nInc", 1), m3d.CRIT_RESIDUAL)
     p, st = s.profile(), s.stats()
-    names = PASS_NAMES_2 if st["passes_per_sweep"] == 2 else PASS_NAMES
+    names = pass_names(sweep_of(st["passes_per_sweep"], w["kind"]))
     out = {"workload": args.workload, "solves": max(args.steps, 1), "passes_per_sweep": st["passes_per_sweep"],
            "sweeps_fp32": p["n_fp32"], "sweeps_fp64": p["n_fp64"]}
     for tag, n, ms, pms in (("fp32", p["n_fp32"], p["ms_fp32"], p["pass_ms_fp32"]),
@@ -975,7 +994,7 @@ def profile_passes(args, w):
         if n:
             out[f"sweep_us_{tag}"] = 1000 * ms / n
             # the refinement's FP64 defect sweeps run the five passes
-            nm = names if (tag == "fp32" or w["precision"] == "fp64") else PASS_NAMES
+            nm = names if (tag == "fp32" or w["precision"] == "fp64") else pass_names("five")
             out[f"pass_us_{tag}"] = {nm[q]: 1000 * pms[q] / n for q in range(5) if nm[q]}
     s.close()
     return out
@@ -1152,7 +1171,7 @@ def run_single(args, w, name, rank, world, local, emit=True, light=False):
     ms64 = max_over_ranks(r64["ms"])
     val64 = V * sum_over_ranks(r64["sweeps"]) / (ms64 / 1000.0)
 
-    # ---- roofline: one sweep (5 FFT passes + fused physics) is the unit -----
+    # ---- roofline: one sweep (its FFT passes + fused physics) is the unit ---
     peaks_path = os.path.join(ROOT, "MEASURED_PEAKS.json")
     if os.path.exists(peaks_path):
         peak = json.load(open(peaks_path))["hbm_gbs"]
@@ -1179,18 +1198,18 @@ def run_single(args, w, name, rank, world, local, emit=True, light=False):
         if n and sum(pms) > 0:
             p = int(np.argmax(pms))
             wb = 4 if fp32 else 8
-            two = pres["st"]["passes_per_sweep"] == 2
-            names, kernels = (PASS_NAMES_2, PASS_KERNELS_2) if two else (PASS_NAMES, PASS_KERNELS)
+            sweep = sweep_of(pres["st"]["passes_per_sweep"], w["kind"])
+            names = pass_names(sweep)
             forcing = w["precision"] == "fp32_refine" and fp32  # inner sweeps read the FP32 defect
-            pb = pass_bytes(c, wb, N, forcing, two)[p]
+            pb = pass_bytes(c, wb, N, forcing, sweep)[p]
             us = 1000 * pms[p] / n
             tr = MEASURED_TRAFFIC.get((name, names[p], wb))
-            kern = {"bound": "hbm", "kernel": kernels[p], "pass": names[p],
+            kern = {"bound": "hbm", "kernel": SWEEP_PASSES[sweep][p][1], "pass": names[p],
                     "achieved": pb / (us * 1e-6) / 1e9, "peak": peak, "unit": "GB/s",
                     "frac": pb / (us * 1e-6) / 1e9 / peak, "traffic": tr[0] if tr else None,
                     "traffic_source": tr[1] if tr else None, "peak_source": peak_src,
                     "bytes_per_launch": pb, "launch_us": us, "share_of_sweep": pms[p] / sum(pms),
-                    "passes_per_sweep": 2 if two else 5,
+                    "passes_per_sweep": pres["st"]["passes_per_sweep"],
                     "pass_us": {names[q]: 1000 * pms[q] / n for q in range(5) if names[q]}}
 
     # ---- error of the timed solve against the FP64 GPU solve at 1e-10 ------
