@@ -11,8 +11,9 @@
 // line_inv is the transposed algorithm and maps spectral -> natural, so a
 // forward + pointwise + inverse sequence needs no reordering at all.
 // The in-register DFTs are mixed-radix (2, 3, 4, 5, 8) decimation in time
-// with every index a compile-time constant; twiddles are read from the
-// per-line table tw[m] = exp(-2 pi i m / N) held in shared memory.
+// with every index a compile-time constant.  Their own twiddles are immediates
+// (rot_const; of the 32-point DFT from the table), the w_N twiddles are read from
+// the per-line table tw[m] = exp(-2 pi i m / N) held in shared memory.
 #pragma once
 #include "fft_smem.cuh"
 

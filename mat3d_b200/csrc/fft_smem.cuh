@@ -29,6 +29,7 @@
 namespace m3d {
 
 constexpr int kMaxStages = 12;
+constexpr int kSMs = 148;  // of a B200: what launch grids and their rules count in
 
 // x / d for 0 <= x, 1 <= d with x * d < 2^32 (always true for indices of a
 // shared-memory tile): round-up reciprocal m = ceil(2^32 / d), q = hi32(x m).
@@ -328,7 +329,7 @@ __device__ __forceinline__ void butterfly(const C2* __restrict__ src, C2* __rest
     for (int r = 0; r < R; ++r) dst[(idx + r * S.Ns.d) * es] = v[r];
 }
 
-// Odd radix R >= 5, compile time: inputs j and R-j are paired
+// Odd prime radix R >= 7, compile time: inputs j and R-j are paired
 // (a_j = x_j + x_{R-j}, b_j = x_j - x_{R-j}) so outputs k and R-k share one set
 // of products:
 //   y_k, y_{R-k} = x_0 + sum_j a_j cos(2 pi jk/R) +- i sign sum_j b_j sin(2 pi jk/R)
@@ -371,9 +372,9 @@ __device__ __forceinline__ void butterfly_odd(const C2* __restrict__ src, C2* __
         T px = x0.x, py = x0.y, qx = 0, qy = 0;
 #pragma unroll
         for (int q = 1; q <= h; ++q) {
-            const int m = (q * k) % R;  // 0 only for a composite R (e.g. 3 * 3 for R = 9)
-            const T cc = m == 0 ? (T)1 : (m <= h ? c[m - 1] : c[R - m - 1]);
-            const T ss = m == 0 ? (T)0 : (m <= h ? sn[m - 1] : -sn[R - m - 1]);
+            const int m = (q * k) % R;  // never 0: R is prime
+            const T cc = m <= h ? c[m - 1] : c[R - m - 1];
+            const T ss = m <= h ? sn[m - 1] : -sn[R - m - 1];
             px += a[q - 1].x * cc;
             py += a[q - 1].y * cc;
             qx += b[q - 1].x * ss;
@@ -421,7 +422,8 @@ struct LineLayout {
 // need); any other radix runs the run-time generic butterfly.
 // one Stockham stage of radix R over every line of the tile (R fixed at
 // compile time, so the loop body is one straight-line butterfly); KIND 0 =
-// butterfly (2, 3, 4, 8), 1 = butterfly_odd, 2 = run-time generic
+// butterfly (radices of 2, 3 and 5 up to 16), 1 = butterfly_odd (primes from 7), 2 =
+// run-time generic
 template <typename C2, int R, int KIND>
 __device__ __forceinline__ void run_stage(const C2* a, C2* b, const C2* tw, const StageIdx& S, int Rrt,
                                           const LineLayout& L, const FastDiv& dl, const FastDiv& dg, int sign) {
@@ -442,7 +444,6 @@ __device__ __forceinline__ void run_stage(const C2* a, C2* b, const C2* tw, cons
 
 template <typename C2, int MaxR = 5>
 __device__ __forceinline__ C2* fft_lines(C2* a, C2* b, const C2* tw, const LinePlan& p, const LineLayout& L, int sign) {
-    const int n = p.n;
     FastDiv dl, dg;  // by the lines of the tile, by the lines of a group
     dl.init(L.nlines);
     dg.init(L.lpg);

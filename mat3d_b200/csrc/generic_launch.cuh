@@ -8,7 +8,8 @@
 // run-time butterfly, whose inputs live in local memory.  So a length takes the
 // smallest variant that holds all its radices.  Measured: FP64 thermal 65^3
 // (65 = 5 x 13) 6.81 -> 3.12 ms a solve (1.8 with fewer stages and the stage
-// constants of fft_smem.cuh), 28^3 (radix 7) batch homogenization 17.7 -> 11.9 ms; lengths of radices up to 5 run the kernel they ran.
+// constants of fft_smem.cuh), 28^3 (radix 7) batch homogenization 17.7 -> 11.9 ms.
+// Lengths of the factors 2, 3 and 5 run the radix-5 variant.
 // The radix-13 and radix-31 variants are instantiated in generic_r13.cu and
 // generic_r31.cu, compiled beside solver.cu.
 #pragma once

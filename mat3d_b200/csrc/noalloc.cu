@@ -193,7 +193,7 @@ extern "C" int m3d_thermal_solve_noalloc(int Nx, int Ny, int Nz, double km, doub
     // what must start at zero: the completion counter and the id sum
     NA_CUDA(cudaMemsetAsync(counter, 0, sizeof(int), stream));
     NA_CUDA(cudaMemsetAsync(idsum, 0, sizeof(unsigned long long), stream));
-    k_noalloc_phase<<<296, 256, 0, stream>>>(d_phase, ph, g.V, idsum);
+    k_noalloc_phase<<<2 * kSMs, 256, 0, stream>>>(d_phase, ph, g.V, idsum);
     NA_CUDA(cudaGetLastError());
     unsigned long long ids = 0;
     NA_CUDA(cudaMemcpyAsync(&ids, idsum, sizeof(ids), cudaMemcpyDeviceToHost, stream));
@@ -246,7 +246,7 @@ extern "C" int m3d_thermal_solve_noalloc(int Nx, int Ny, int Nz, double km, doub
     NA_CUDA(cudaMemcpyAsync(mats, hm, sizeof(hm), cudaMemcpyHostToDevice, stream));
     NA_CUDA(cudaMemcpyAsync(tw, htw.data(), htw.size() * sizeof(double2), cudaMemcpyHostToDevice, stream));
     NA_CUDA(cudaMemcpyAsync(ctl, &hc, sizeof(hc), cudaMemcpyHostToDevice, stream));
-    k_noalloc_fill<<<296, 256, 0, stream>>>(d_grad, g.V, E[0], E[1], E[2]);
+    k_noalloc_fill<<<2 * kSMs, 256, 0, stream>>>(d_grad, g.V, E[0], E[1], E[2]);
 
     ProMat<double, C> pro{ph, d_grad, g.V, mats, 2, nullptr};
     SpecGreen<double, C> sg;
@@ -293,7 +293,7 @@ extern "C" int m3d_thermal_solve_noalloc(int Nx, int Ny, int Nz, double km, doub
         if (hc.done) break;
     }
     if (scheme == 2) {
-        k_noalloc_to_grad<<<296, 256, 0, stream>>>(d_grad, ph, g.V, 1.0 / ki, 1.0 / km);
+        k_noalloc_to_grad<<<2 * kSMs, 256, 0, stream>>>(d_grad, ph, g.V, 1.0 / ki, 1.0 / km);
         NA_CUDA(cudaGetLastError());
         NA_CUDA(cudaStreamSynchronize(stream));
     }

@@ -265,9 +265,11 @@ constexpr size_t xturn_cp_smem() {
 // warps of more than 170 registers run one CTA per SM: uncapped the long FP64
 // lines take 176-220 and FP32 256 points 185.  Measured per launch, six
 // components: FP64 256^3 887 us uncapped, 625 at two CTAs (no spill), 599 at
-// three (116 bytes); FP32 256^3 531, 398, 425 (200 bytes).  FP32 96^3 three
-// (140 bytes of spill; 157 -> 142 ms of a batch group's x turnaround), FP64 96^3
-// two.  Three warps of 178-236 registers: four CTAs of 168.
+// three (116 bytes); FP32 256^3 531, 398, 425 (200 bytes); FP64 128^3 110, 82, 82; FP64
+// 96^3 51, 43, 60 (one entry).  FP32 96^3 three (140 bytes of spill; 157 -> 142 ms of a
+// batch group's x turnaround).  Three warps of 178-236 registers: FP32 256^3 263 us
+// uncapped, 190 at three or four CTAs, FP64 256^3 399, 296, 296, the reference rule's
+// check at FP64 96^3 29, 25, 26; four CTAs of 168 registers.
 template <typename T, int N, int C> struct XcpMinB {
     static constexpr int value = C == 3 ? ((N == 256 || (sizeof(T) == 8 && N >= 96)) ? 4 : 1)
                                         : (sizeof(T) == 8 && N >= 128) ? 3

@@ -56,7 +56,13 @@ template <typename T, int N> struct PlaneGeom {
         static constexpr int CPC = CPC_, CS = 6 / CPC_, NT = NT_, MINB = MINB_, NW = NT_ / 32;  \
         static constexpr size_t smem() { return (size_t)(CPC * NN * NN + NN) * 2 * sizeof(TY); } \
     };
-// components per CTA, threads, CTAs per SM
+// components per CTA, threads, CTAs per SM.  Others, us per k_plane launch (these ->
+// other): FP32 32^3 x 144 entries 77 -> 85 (3, 128, 8), 80 (6, 192, 4); 48^3 x 96 169 ->
+// 166 (3, 192, 4), 169 (6, 256, 2); 64^3 x 48 193 -> 189 (6, 512, 1), 220 (2, 192, 3); 96^3
+// x 24 411 -> 480 (2, 384, 1), 454 (1, 256, 3).  FP64, one entry and 96, 48 or 24: 32^3 18
+// and 91 -> 16 and 96 (3, 128, 4), 19 and 94 (6, 384, 2); 48^3 25 and 186 -> 35 and 207
+// (6, 512, 1), 21 and 184 (2, 192, 3); 64^3 28 and 221 -> 27 and 277 (2, 256, 1), 29 and
+// 229 (1, 192, 3).
 M3D_PLANE(float, 32, 6, 256, 4)
 M3D_PLANE(float, 48, 6, 384, 2)
 M3D_PLANE(float, 64, 3, 256, 2)

@@ -1,4 +1,4 @@
-// passes_zmid.cuh -- the fused z pass of five-pass sweeps: z inverse, the
+// passes_zmid.cuh -- the fused z pass of four-pass sweeps: z inverse, the
 // pointwise middle of the sweep (mid_ops.cuh) and the next sweep's z forward in
 // one kernel, on the row layout of the half spectrum (passes.cuh).
 //
@@ -49,7 +49,7 @@ template <typename T, int N, int C> struct ZRowsGeom {
         return (size_t)N * 2 * sizeof(T) + NBUF * tile_bytes + Op::smem_bytes(nph);
     }
 };
-constexpr int kZRowsGrid = 148 * 4;
+constexpr int kZRowsGrid = kSMs * 4;
 
 // CTAs (of three warps) per SM: four, 168 registers.  The inelastic kernels spill
 // 100-400 bytes under it; at 128 registers (five CTAs, one buffer) FP64 256^3
@@ -327,6 +327,6 @@ __global__ void __launch_bounds__(256)
     block_reduce_store<Op::NSUM>(acc, red, partials, b, gridDim.x, blockIdx.x);
     fused_finalize(fin, ctl, partials, Op::NSUM, b);
 }
-constexpr int kZGenGrid = 148 * 8;  // CTAs per entry at most (partial sums, as kZRowsGrid)
+constexpr int kZGenGrid = kSMs * 8;  // CTAs per entry at most (partial sums, as kZRowsGrid)
 
 }  // namespace m3d

@@ -732,7 +732,7 @@ struct m3d_rec {
     size_t y_smem() const { return (size_t)Ny * 16 + 3 * (size_t)Ny * TZ * 16; }
     size_t x_smem() const { return (size_t)Nx * 16 + 3 * (size_t)Nx * TZX * 16 + 2 * (size_t)Nx * TZX * 8; }
     size_t xr_smem() const { return (size_t)Nx * 16 + 3 * (size_t)Nx * TZX * 16; }
-    int grid1d() const { return (int)std::min<long long>(148 * 8, (xyz + kThreads - 1) / kThreads); }
+    int grid1d() const { return (int)std::min<long long>(kSMs * 8, (xyz + kThreads - 1) / kThreads); }
 
     // the kernels of one pass, in order; `prof` brackets each with events
     template <int MaxR>
@@ -978,7 +978,7 @@ struct m3d_rec {
         *h_ctl = c;
         MR_CUDA(cudaMemcpyAsync(d_ctl, h_ctl, sizeof(RecCtl), cudaMemcpyHostToDevice, stream));
         MR_CUDA(cudaMemsetAsync(thr, 0, offsetof(ThrBins, k), stream));
-        const int grid = (int)std::min<long long>(148 * 4, (xyz + kHistThreads - 1) / kHistThreads);
+        const int grid = (int)std::min<long long>(kSMs * 4, (xyz + kHistThreads - 1) / kHistThreads);
         krec_thr_hist<<<grid, kHistThreads, 0, stream>>>(m, thr, xyz);
         krec_thr_walk<<<1, kHistThreads, 0, stream>>>(thr, d_ctl, xyz);
         krec_thr_apply<<<grid1d(), kThreads, 0, stream>>>(m, d_ctl, xyz);

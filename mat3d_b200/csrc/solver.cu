@@ -713,7 +713,7 @@ void m3d_solver::pass_y(int sign, int CC, Ctl* ctl, typename Cx<T>::t* sp) {
             const int ntiles = CC * gridB() * Nx * ntz;
             auto kern = sign < 0 ? k_ypass_tma<T, NN, -1> : k_ypass_tma<T, NN, +1>;
             allow_smem(kern);
-            int per_sm = 1, dev = 0, nsm = 148;
+            int per_sm = 1, dev = 0, nsm = kSMs;
             cudaGetDevice(&dev);
             cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
             cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kFastThreads, Y::smem());
@@ -762,7 +762,7 @@ int m3d_solver::pass_x(Spec op, Ctl* ctl, typename Cx<T>::t* sp) {
                 // the warps of k_xturn_r1 fill the chip (the six-transform kernel, ahead
                 // by 2% at 576, was behind by 4% at 864 and 10% at 1728).
                 if constexpr (NN <= 96) {
-                    if (use_xcp && NN >= 32 && (long long)B * Ny * ngrp <= 5 * 148) {
+                    if (use_xcp && NN >= 32 && (long long)B * Ny * ngrp <= 5 * kSMs) {
                         nblk = Ny * ngrp;
                         allow_smem(k_xturn_r1cp<T, NN>);
                         k_xturn_r1cp<T, NN><<<dim3(nblk, gridB()), 96, xturn_r1cp_smem<T, NN>(), stream>>>(g, tw<T>(0), sp, op, ctl);
@@ -775,7 +775,7 @@ int m3d_solver::pass_x(Spec op, Ctl* ctl, typename Cx<T>::t* sp) {
                         auto kern = k_xturn_r1_tma<T, NN>;
                         allow_smem(kern);
                         static const int slots = [kern] {  // resident CTAs per SM x SMs
-                            int per_sm = 1, dev = 0, nsm = 148;
+                            int per_sm = 1, dev = 0, nsm = kSMs;
                             cudaGetDevice(&dev);
                             cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
                             cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kXRegWarps * 32, X::smem());
@@ -1934,7 +1934,7 @@ int m3d_solver::load_phase(int r, const int32_t* phase, int nph, std::vector<lon
     M3D_CUDA(cudaMemsetAsync(d_pstat + kMaxPhases + 1, 0xff, sizeof(unsigned long long), stream));
     int32_t* ids = (int32_t*)d_spec;
     M3D_CUDA(cudaMemcpyAsync(ids, phase, (size_t)V * sizeof(int32_t), cudaMemcpyHostToDevice, stream));
-    const int nblk = (int)std::min<long long>((V + 255) / 256, 148 * 8);
+    const int nblk = (int)std::min<long long>((V + 255) / 256, kSMs * 8);
     k_phase_in<<<nblk, 256, 0, stream>>>(ids, d_phase + (size_t)r * V, V, nph, d_pstat);
     M3D_CUDA(cudaGetLastError());
     unsigned long long hs[kMaxPhases + 2];
@@ -2187,7 +2187,7 @@ static __global__ void k_means_sum(const double* __restrict__ part, int NS, int 
 // launches and one copy for all of them.  (A launch, a copy and a host sum per
 // entry took 30 us each, 4.4 of 21 ms of a homogenization of 24 RVEs at 32^3.)
 static int entry_sums(m3d_solver* h, int b0, int nb, double* sums) {
-    const int C = h->C, nblk = 296;
+    const int C = h->C, nblk = 2 * kSMs;
     double* part = h->d_part;
     double* tot = part + (size_t)nb * 2 * C * nblk;
     if (h->part_cap < (size_t)nb * 2 * C * (nblk + 1)) return fail(M3D_ERR_STATE, "partials buffer too small");

@@ -402,7 +402,7 @@ struct m3d_solver2d {
     // 25 iterations took 3.58 -> 1.73 ms at 64^2, 3.42 -> 3.01 at 171^2, 6.8 -> 4.5 at
     // 512^2, 23.9 -> 15.4 at 1024^2 (with the columns' tiles).
     void pick_mid() {
-        g_mid = std::max(1, std::min(std::min(16, (int)(48 * 1024 / (48 * (size_t)Ny))), Nx / 296));
+        g_mid = std::max(1, std::min(std::min(16, (int)(48 * 1024 / (48 * (size_t)Ny))), Nx / (2 * kSMs)));
         g_mid -= g_mid % 2 == 0;
         if (mid_smem() > 220 * 1024) g_mid = 0;
         nt_mid = plan_threads(py, 3 * std::max(1, g_mid));

@@ -57,7 +57,7 @@ __global__ void k_colsum(const TX* __restrict__ x, int C, int b, long long V, do
 
 template <typename TX>
 static int colsum_mean(m3d_solver* h, const void* x, int C, int b, double* out) {
-    const int nblk = 296;
+    const int nblk = 2 * kSMs;
     k_colsum<TX><<<nblk, 256, 0, h->stream>>>((const TX*)x, C, b, h->g.V, h->d_part);
     h->st.kernel_launches += 1;
     M3D_CUDA(cudaGetLastError());

@@ -28,8 +28,9 @@ cudaError_t go(int entries, cudaStream_t st, const GridDims& g, const typename C
 }  // namespace
 
 // The EM kernels are for the shapes that the two-pass sweeps (passes_plane.cuh,
-// passes_slab.cuh) do not cover; at 96 points and below five passes remain only
-// for non-cubic grids.
+// passes_slab.cuh) do not cover.  Of those, five passes remain for lines of 32, 48
+// and 64 points, of 96 in FP32, and of 128 in FP32 thermal solves: grids whose other
+// lengths keep them from two passes.
 template <typename T, int C, class F> void with_em_n(int n, F&& f) {
     switch (n) {
         case 96: if constexpr (sizeof(T) == 8) f(IntC<96>{}); break;
