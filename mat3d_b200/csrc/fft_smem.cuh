@@ -218,46 +218,9 @@ __device__ __forceinline__ void dft_small(C2 (&v)[R], const C2* tw, int n, int s
         v[4] = mk<C2>(t1.x + u1.y, t1.y - u1.x);
         v[2] = mk<C2>(t2.x - u2.y, t2.y + u2.x);
         v[3] = mk<C2>(t2.x + u2.y, t2.y - u2.x);
-    } else if constexpr (R == 9) {
-        // inputs m and 9 - m paired (see butterfly_odd): about the operations of two
-        // rounds of 3-point DFTs with w_9 twiddles between them, which rounded more
-        // (FP64 transforms of 27, 81, 171 and 729 points 4, 10, 9 and 19% further from
-        // their exact values); solves at lengths of nines take 0 to 2% longer
-        const T cs[9] = {(T)1, (T)0.766044443118978035202392650555417L, (T)0.173648177666930348851716626769315L, (T)-0.5,
-                         (T)-0.939692620785908384054109277324731L, (T)-0.939692620785908384054109277324731L, (T)-0.5,
-                         (T)0.173648177666930348851716626769315L, (T)0.766044443118978035202392650555417L};
-        const T sn[9] = {(T)0, (T)0.642787609686539326322643409907263L, (T)0.984807753012208059366743024589523L,
-                         (T)0.866025403784438646763723170752936L, (T)0.342020143325668733044099614682260L,
-                         (T)-0.342020143325668733044099614682260L, (T)-0.866025403784438646763723170752936L,
-                         (T)-0.984807753012208059366743024589523L, (T)-0.642787609686539326322643409907263L};
-        C2 a[4], b[4], out[8];
-        C2 sum = v[0];
-#pragma unroll
-        for (int m = 1; m < 5; ++m) {
-            a[m - 1] = cadd(v[m], v[9 - m]);
-            b[m - 1] = csub(v[m], v[9 - m]);
-            sum = cadd(sum, a[m - 1]);
-        }
-#pragma unroll
-        for (int k = 1; k < 5; ++k) {
-            C2 A = v[0], B = mk<C2>(0, 0);
-#pragma unroll
-            for (int m = 1; m < 5; ++m) {
-                const T c = cs[k * m % 9], d = sign < 0 ? -sn[k * m % 9] : sn[k * m % 9];
-                A.x += c * a[m - 1].x;
-                A.y += c * a[m - 1].y;
-                B.x += d * b[m - 1].x;
-                B.y += d * b[m - 1].y;
-            }
-            out[k - 1] = mk<C2>(A.x - B.y, A.y + B.x);
-            out[8 - k] = mk<C2>(A.x + B.y, A.y - B.x);
-        }
-        v[0] = sum;
-#pragma unroll
-        for (int k = 1; k < 9; ++k) v[k] = out[k - 1];
-    } else if constexpr (R == 16) {
-        // 4 x 4: w_16 twiddles between two rounds of 4-point DFTs
-        constexpr int P = 4;
+    } else if constexpr (R == 9 || R == 16) {
+        // R = P x P: w_R twiddles between two rounds of P-point DFTs
+        constexpr int P = R == 9 ? 3 : 4;
         C2 sub[P][P];
 #pragma unroll
         for (int p = 0; p < P; ++p) {
@@ -269,7 +232,21 @@ __device__ __forceinline__ void dft_small(C2 (&v)[R], const C2* tw, int n, int s
         for (int k1 = 0; k1 < P; ++k1) {
             C2 t[P];
 #pragma unroll
-            for (int p = 0; p < P; ++p) t[p] = p == 0 || k1 == 0 ? sub[p][k1] : rot_const<C2, 16>(sub[p][k1], p * k1, sign);
+            for (int p = 0; p < P; ++p) {
+                if (p == 0 || k1 == 0) {
+                    t[p] = sub[p][k1];
+                } else if constexpr (R == 16) {
+                    t[p] = rot_const<C2, 16>(sub[p][k1], p * k1, sign);
+                } else {  // cos and sin of 40, 80 and 160 degrees
+                    const T c = p * k1 == 1 ? (T)0.766044443118978035202392650555417L
+                                            : (p * k1 == 2 ? (T)0.173648177666930348851716626769315L
+                                                           : (T)-0.939692620785908384054109277324731L);
+                    const T sn = p * k1 == 1 ? (T)0.642787609686539326322643409907263L
+                                             : (p * k1 == 2 ? (T)0.984807753012208059366743024589523L
+                                                            : (T)0.342020143325668733044099614682260L);
+                    t[p] = cmul(sub[p][k1], mk<C2>(c, sign < 0 ? -sn : sn));
+                }
+            }
             dft_small<C2, P>(t, tw, n, sign);
 #pragma unroll
             for (int k2 = 0; k2 < P; ++k2) v[k1 + P * k2] = t[k2];
@@ -311,9 +288,53 @@ __device__ __forceinline__ void dft_small(C2 (&v)[R], const C2* tw, int n, int s
     }
 }
 
+// 9-point DFT as paired sums, inputs m and 9 - m together (see butterfly_odd): about
+// the operations of the two rounds of 3-point DFTs of dft_small, and a single
+// transform of 27, 81, 171 or 729 points is 4, 10, 9 or 19% nearer its exact values
+// with it.  The reconstruction, which offers plain transforms, takes it.  The solvers
+// do not: their forward and inverse transforms undo each other's rounding better with
+// the 3-point rounds (FP64 strains of thermal 27^3 and 81^3 12 and 17% nearer the
+// 64-bit results, of plane 81^2, 243^2 and 486^2 24, 23 and 22%).
+template <typename C2>
+__device__ __forceinline__ void dft9_paired(C2 (&v)[9], int sign) {
+    typedef decltype(C2().x) T;
+    const T cs[9] = {(T)1, (T)0.766044443118978035202392650555417L, (T)0.173648177666930348851716626769315L, (T)-0.5,
+                     (T)-0.939692620785908384054109277324731L, (T)-0.939692620785908384054109277324731L, (T)-0.5,
+                     (T)0.173648177666930348851716626769315L, (T)0.766044443118978035202392650555417L};
+    const T sn[9] = {(T)0, (T)0.642787609686539326322643409907263L, (T)0.984807753012208059366743024589523L,
+                     (T)0.866025403784438646763723170752936L, (T)0.342020143325668733044099614682260L,
+                     (T)-0.342020143325668733044099614682260L, (T)-0.866025403784438646763723170752936L,
+                     (T)-0.984807753012208059366743024589523L, (T)-0.642787609686539326322643409907263L};
+    C2 a[4], b[4], out[8];
+    C2 sum = v[0];
+#pragma unroll
+    for (int m = 1; m < 5; ++m) {
+        a[m - 1] = cadd(v[m], v[9 - m]);
+        b[m - 1] = csub(v[m], v[9 - m]);
+        sum = cadd(sum, a[m - 1]);
+    }
+#pragma unroll
+    for (int k = 1; k < 5; ++k) {
+        C2 A = v[0], B = mk<C2>(0, 0);
+#pragma unroll
+        for (int m = 1; m < 5; ++m) {
+            const T c = cs[k * m % 9], d = sign < 0 ? -sn[k * m % 9] : sn[k * m % 9];
+            A.x += c * a[m - 1].x;
+            A.y += c * a[m - 1].y;
+            B.x += d * b[m - 1].x;
+            B.y += d * b[m - 1].y;
+        }
+        out[k - 1] = mk<C2>(A.x - B.y, A.y + B.x);
+        out[8 - k] = mk<C2>(A.x + B.y, A.y - B.x);
+    }
+    v[0] = sum;
+#pragma unroll
+    for (int k = 1; k < 9; ++k) v[k] = out[k - 1];
+}
+
 // butterfly j of a stage: inputs j + r nb, twiddles w^(k r step) with
 // j = g Ns + k, outputs g Ns R + k + r Ns
-template <typename C2, int R>
+template <typename C2, int R, bool Paired9 = false>
 __device__ __forceinline__ void butterfly(const C2* __restrict__ src, C2* __restrict__ dst, int j, int g, int k,
                                           const StageIdx& S, int es, const C2* tw, int sign) {
     C2 v[R];
@@ -323,7 +344,8 @@ __device__ __forceinline__ void butterfly(const C2* __restrict__ src, C2* __rest
 #pragma unroll
         for (int r = 1; r < R; ++r) v[r] = cmul(v[r], twid(tw, k * r * S.step, sign));
     }
-    dft_small<C2, R>(v, tw, S.nb.d * R, sign);
+    if constexpr (R == 9 && Paired9) dft9_paired(v, sign);
+    else dft_small<C2, R>(v, tw, S.nb.d * R, sign);
     const int idx = g * S.Ns.d * R + k;
 #pragma unroll
     for (int r = 0; r < R; ++r) dst[(idx + r * S.Ns.d) * es] = v[r];
@@ -423,7 +445,7 @@ struct LineLayout {
 // one Stockham stage of radix R over every line of the tile (R fixed at
 // compile time, so the loop body is one straight-line butterfly); KIND 0 =
 // butterfly (radices of 2, 3 and 5 up to 16), 1 = butterfly_odd (primes from 7), 2 =
-// run-time generic
+// run-time generic, 3 = butterfly with the paired 9-point DFT
 template <typename C2, int R, int KIND>
 __device__ __forceinline__ void run_stage(const C2* a, C2* b, const C2* tw, const StageIdx& S, int Rrt,
                                           const LineLayout& L, const FastDiv& dl, const FastDiv& dg, int sign) {
@@ -436,13 +458,13 @@ __device__ __forceinline__ void run_stage(const C2* a, C2* b, const C2* tw, cons
         const int grp = dg.div(line);
         const int base = grp * L.gstride + (line - grp * L.lpg) * L.lstride;
         const int g = S.Ns.div(j), k = j - g * S.Ns.d;
-        if constexpr (KIND == 0) butterfly<C2, R>(a + base, b + base, j, g, k, S, es, tw, sign);
+        if constexpr (KIND == 0 || KIND == 3) butterfly<C2, R, KIND == 3>(a + base, b + base, j, g, k, S, es, tw, sign);
         else if constexpr (KIND == 1) butterfly_odd<C2, R>(a + base, b + base, j, g, k, S, es, tw, sign);
         else butterfly_generic<C2>(a + base, b + base, Rrt, j, g, k, S, es, tw, sign);
     }
 }
 
-template <typename C2, int MaxR = 5>
+template <typename C2, int MaxR = 5, bool Paired9 = false>
 __device__ __forceinline__ C2* fft_lines(C2* a, C2* b, const C2* tw, const LinePlan& p, const LineLayout& L, int sign) {
     FastDiv dl, dg;  // by the lines of the tile, by the lines of a group
     dl.init(L.nlines);
@@ -457,7 +479,7 @@ __device__ __forceinline__ C2* fft_lines(C2* a, C2* b, const C2* tw, const LineP
             case 5: run_stage<C2, 5, 0>(a, b, tw, S, R, L, dl, dg, sign); break;
             case 6: run_stage<C2, 6, 0>(a, b, tw, S, R, L, dl, dg, sign); break;
             case 8: run_stage<C2, 8, 0>(a, b, tw, S, R, L, dl, dg, sign); break;
-            case 9: run_stage<C2, 9, 0>(a, b, tw, S, R, L, dl, dg, sign); break;
+            case 9: run_stage<C2, 9, Paired9 ? 3 : 0>(a, b, tw, S, R, L, dl, dg, sign); break;
             case 10: run_stage<C2, 10, 0>(a, b, tw, S, R, L, dl, dg, sign); break;
             case 12: run_stage<C2, 12, 0>(a, b, tw, S, R, L, dl, dg, sign); break;
             case 15: run_stage<C2, 15, 0>(a, b, tw, S, R, L, dl, dg, sign); break;

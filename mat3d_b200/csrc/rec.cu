@@ -205,7 +205,7 @@ __global__ void __launch_bounds__(kThreads) krec_z(double2* __restrict__ A, doub
         const int nxt = tile + gridDim.x;
         if (nxt < ntiles) fetch(B[f], nxt);
         cp_async_commit();
-        double2* r = fft_lines<double2, MaxR>(B[d], B[d == 2 ? 0 : d + 1], tw, pz, L,
+        double2* r = fft_lines<double2, MaxR, true>(B[d], B[d == 2 ? 0 : d + 1], tw, pz, L,
                                               (MODE == Z_INV || MODE == Z_BWD) ? +1 : -1);
         if (MODE == Z_INV) {
             cp_async_wait_group1();  // the old field landed (the next tile may still be in flight)
@@ -307,7 +307,7 @@ __global__ void __launch_bounds__(kThreads) krec_y(double2* __restrict__ A, cons
         const int nxt = tile + gridDim.x;
         if (nxt < ntiles) col_fetch(B[f], A, tile_of(nxt), Ny, TZ, dz);
         cp_async_commit();
-        const double2* r = fft_lines<double2, MaxR>(B[d], B[d == 2 ? 0 : d + 1], tw, py, L, MODE == Y_INV ? +1 : -1);
+        const double2* r = fft_lines<double2, MaxR, true>(B[d], B[d == 2 ? 0 : d + 1], tw, py, L, MODE == Y_INV ? +1 : -1);
         col_store(A, r, tile_of(tile), Ny, TZ, dz);
         d = f;
     }
@@ -352,7 +352,7 @@ __global__ void __launch_bounds__(kThreads) krec_xout(double2* __restrict__ A, d
         const int nxt = tile + gridDim.x;
         if (nxt < ntiles) col_fetch(B[f], A, tile_of(nxt), Nx, TZ, dz);
         cp_async_commit();
-        const double2* r = fft_lines<double2, MaxR>(B[d], B[d == 2 ? 0 : d + 1], tw, px, L, sign);
+        const double2* r = fft_lines<double2, MaxR, true>(B[d], B[d == 2 ? 0 : d + 1], tw, px, L, sign);
         const ColTile c = tile_of(tile);
         if (OUT == XO_COPY) {
             col_store(A, r, c, Nx, TZ, dz);
@@ -429,7 +429,7 @@ __global__ void __launch_bounds__(kThreads) krec_xturn(double2* __restrict__ A, 
         const int nxt = tile + gridDim.x;
         if (nxt < ntiles) fetch(B[f], NB[nbi ^ 1], nxt);
         cp_async_commit();
-        double2* r = fft_lines<double2, MaxR>(B[d], B[d == 2 ? 0 : d + 1], tw, px, L, -1);
+        double2* r = fft_lines<double2, MaxR, true>(B[d], B[d == 2 ? 0 : d + 1], tw, px, L, -1);
         double2* o = (r == B[d]) ? B[d == 2 ? 0 : d + 1] : B[d];
         const ColTile c = tile_of(tile);
         const double* nct = NB[nbi];
@@ -456,7 +456,7 @@ __global__ void __launch_bounds__(kThreads) krec_xturn(double2* __restrict__ A, 
             }
         }
         __syncthreads();
-        const double2* q = fft_lines<double2, MaxR>(r, o, tw, px, L, +1);
+        const double2* q = fft_lines<double2, MaxR, true>(r, o, tw, px, L, +1);
         col_store(A, q, c, Nx, TZ, dz);
         d = f;
         nbi ^= 1;
