@@ -98,7 +98,7 @@ typedef struct {
     double k0;               /* reference conductivity (thermal) */
     double vol_fraction[16]; /* per phase id */
     long long kernel_launches; /* kernels this handle launched since creation */
-    int passes_per_sweep;    /* launches per linear sweep of the last run: 5 (z, y, x, y, z passes),
+    int passes_per_sweep;    /* launches per sweep of the last run: 5 (z, y, x, y, z passes),
                                 4 (the z passes fused with the next sweep's) or 2 (x turnaround + the
                                 y-z slab pass, or kz-plane pass + fused z pass) */
 } m3d_stats;
@@ -179,7 +179,7 @@ typedef struct {
     long long n_fp64;    /* FP64 sweeps timed */
     double ms_fp32;      /* summed device time of FP32 sweeps */
     long long n_fp32;    /* FP32 sweeps timed */
-    /* the same time split by pass (events around each pass of the linear
+    /* the same time split by pass (events around each pass of the
        sweeps): z forward, y forward, x turnaround, y inverse, z inverse; on
        two-pass sweeps (m3d_stats.passes_per_sweep == 2) slot 2 holds the x
        turnaround (kz-plane pass) and slot 4 the y-z slab (fused z) pass, slots
