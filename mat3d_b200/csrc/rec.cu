@@ -1035,7 +1035,7 @@ static int rec_alloc(int Nx, int Ny, int Nz, int device, m3d_rec** out) {
     h->Nx = Nx; h->Ny = Ny; h->Nz = Nz;
     h->xyz = (long long)Nx * Ny * Nz;
     h->device = device;
-    if (!make_plan(Nx, h->px) || !make_plan(Ny, h->py) || !make_plan(Nz, h->pz)) {
+    if (!make_plan(Nx, h->px, 0, true) || !make_plan(Ny, h->py, 0, true) || !make_plan(Nz, h->pz, 0, true)) {
         delete h;
         return failr(M3D_ERR_UNSUPPORTED, "grid sizes need prime factors <= 32");
     }
